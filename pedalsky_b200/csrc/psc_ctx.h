@@ -99,7 +99,7 @@ struct psc_ctx {
   float4* d_bap = nullptr;              // per-view aerial-perspective LUTs
   // voxel-grid form: the grid values as corner quads and the adjoint's
   // gradient as x pairs (GridDev::quads / grad_pairs), grown to the largest
-  // grid seen
+  // grid seen; GridDev::nonfinite lies behind the quads
   float4* d_grid_quads = nullptr;
   float2* d_grad_pairs = nullptr;
   size_t grid_pairs_cap = 0;  // entries of the quad array (the pair array holds as many)

@@ -2477,13 +2477,15 @@ int stage_grid_layout(psc_ctx* c, psc::GridDev& gd, bool adjoint, cudaStream_t s
     dfree(c->d_grid_quads);
     dfree(c->d_grad_pairs);
     c->grid_pairs_cap = 0;
-    PSC_CUDA(cudaMalloc(&c->d_grid_quads, nq * sizeof(float4)), "cudaMalloc grid quads");
+    PSC_CUDA(cudaMalloc(&c->d_grid_quads, (nq + 1u) * sizeof(float4)), "cudaMalloc grid quads");  // + the flag
     PSC_CUDA(cudaMalloc(&c->d_grad_pairs, nq * sizeof(float2)), "cudaMalloc gradient pairs");
     c->grid_pairs_cap = nq;
   }
-  if (psc::launch_grid_quads(gd.values, c->d_grid_quads, gd.nx, gd.ny, gd.nz, s))
+  uint32_t* const nonfinite = reinterpret_cast<uint32_t*>(c->d_grid_quads + c->grid_pairs_cap);
+  if (psc::launch_grid_quads(gd.values, c->d_grid_quads, nonfinite, gd.nx, gd.ny, gd.nz, s))
     return fail(PSC_ERR_CUDA, "grid quad launch failed: %s", cudaGetErrorString(cudaGetLastError()));
   gd.quads = c->d_grid_quads;
+  gd.nonfinite = nonfinite;
   if (adjoint) {
     PSC_CUDA(cudaMemsetAsync(c->d_grad_pairs, 0, np * sizeof(float2), s), "gradient pair reset");
     gd.grad_pairs = c->d_grad_pairs;

@@ -176,14 +176,16 @@ struct GridDev {
   // (x = xk - 1, xk) (grad_pairs), and folds them into grad afterwards
   // (launch_grid_fold)
   const float4* quads;
+  const uint32_t* nonfinite;  // 1 when the grid holds an infinity or NaN
   float2* grad_pairs;
 };
 int launch_grid_march(const MarchUniforms& u, const ViewDev& v, const GridDev& g, bool adjoint,
                       cudaStream_t stream);
 // quads[(y (nz + 1) + zk) (nx + 1) + xk] as GridDev::quads from the ny x nz x
-// nx values
+// nx values; *nonfinite = 1 when a value is an infinity or NaN, else 0
 // grad[r nx + x] += gp[r (nx + 1) + x + 1].x + gp[r (nx + 1) + x].y
-int launch_grid_quads(const float* values, float4* quads, uint32_t nx, uint32_t ny, uint32_t nz, cudaStream_t stream);
+int launch_grid_quads(const float* values, float4* quads, uint32_t* nonfinite, uint32_t nx, uint32_t ny,
+                      uint32_t nz, cudaStream_t stream);
 int launch_grid_fold(const float2* grad_pairs, float* grad, uint32_t nx, uint32_t rows, cudaStream_t stream);
 // d loss / d (base_m, top_m) of layer 0 in the grid form, added to out[0..1]
 // (grid_layer_grad.cu); g.bg / g.target / g.inv_n as for the adjoint.
