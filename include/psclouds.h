@@ -611,7 +611,10 @@ int psc_autotune_steps(psc_ctx* ctx, PscBatchView* views, uint32_t n, float max_
 typedef struct PscDensityGrid {
   const float* values;          /* ny x nz x nx FP32, x fastest, then z, then altitude */
   uint32_t nx, ny, nz;          /* cells along world x (east), altitude, world z (south) */
-  uint32_t checkpoint_every;    /* psc_adjoint: transmittance checkpoint interval, 1..32 steps */
+  uint32_t checkpoint_every;    /* psc_adjoint, psc_layer_gradient: 1..32, at most
+                                   PSC_GRID_MAX_CHECKPOINTS intervals; checked, and without effect
+                                   on the result (the reverse sweep walks the optical depth back
+                                   exactly and needs no checkpoints) */
   float min_x_m, min_z_m;       /* world x / z of the grid's low corner */
   float size_x_m, size_z_m;     /* horizontal extent (altitude extent: layer 0 base..top) */
   float density_scale;          /* multiplies every value */
@@ -631,9 +634,7 @@ int psc_render_grid(psc_ctx* ctx, const PscDensityGrid* grid, const PscView* vie
  * sum((I - target)^2) / (3 * viewport_w * viewport_h), summed over the
  * view's rectangle, so row bands of one viewport add up to the whole
  * image's loss and gradient.  `background` and `target` are device float4
- * per pixel of the rectangle.  The march keeps transmittance at every
- * `checkpoint_every`-th step and recomputes the steps between checkpoints
- * in the reverse sweep.  Results are ADDED to `grad_values` (device, same
+ * per pixel of the rectangle.  Results are ADDED to `grad_values` (device, same
  * shape as the grid), `*grad_density_scale` and `*loss` (device doubles),
  * so callers zero them first; view outputs, if given, receive L and T. */
 int psc_adjoint(psc_ctx* ctx, const PscDensityGrid* grid, const PscView* view,

@@ -14,23 +14,26 @@
 // the forward march takes its light taps and LUT lookups only where the grid
 // is not empty (see `every` in grid_pixel for grids with infinities or NaN).
 //
-// Adjoint: one thread per ray runs the forward march keeping the
-// transmittance at every k-th step, evaluates its pixel's loss term
-// (I - target)^2 / N with I = L + background * T, then walks the checkpoint
-// segments backwards: each segment's primary grid values and their prefix
-// sums are refetched, then the segment is traversed in reverse, carrying the
-// adjoint of the transmittance; the light taps and LUT lookups of a sample
-// are taken there, once.  The transmittance before a
-// step is the checkpoint's times exp(-sigma_t * step * k * prefix).
-// Checkpoints and segment buffers live
-// in dynamic shared memory laid out [slot][thread], so every access is
-// conflict-free and nothing is kept in local memory.  d loss / d density at the primary sample and d loss /
-// d optical depth toward the sun are scattered into the gradient grid with
-// atomic adds over the trilinear weights of the primary sample and of the
-// six light taps.  Loss and d loss / d density_scale are reduced per CTA and
-// added in double.
+// Adjoint: one thread per ray runs the forward march, evaluates its pixel's
+// loss term (I - target)^2 / N with I = L + background * T, then walks the
+// steps backwards, carrying the adjoint of the transmittance.  The
+// transmittance before a step is exp(-sigma_t * step * k * prefix), prefix the
+// sum of the grid values of the steps before it: the forward march sums them
+// in FP64 and the reverse sweep takes each step's value off again, which loses
+// nothing against FP32 values, so neither checkpoints nor a recomputed segment
+// are needed and the L1 has no shared memory to make room for (checkpoints and
+// segment buffers in 25.6 KB of shared memory per CTA: 1886 us, without: 1668
+// us; each KB per CTA more cost about 20 us).  d loss / d density at the
+// primary sample and d loss / d optical depth toward the sun are scattered
+// into the gradient with vector atomic adds over the trilinear weights of the
+// primary sample and of the six light taps, one 16-byte add per y row (as
+// 8-byte pairs, four per tap, the scatter took 270 us of 1668; now 90 of
+// 1362).  Loss and d loss / d density_scale are reduced per CTA and added in
+// double.
 #include <cuda_runtime.h>
 #include <stdint.h>
+
+#include <type_traits>
 
 #include "march_fast_body.cuh"
 
@@ -41,130 +44,172 @@ constexpr int kTileW = 16;
 constexpr int kTileH = 8;
 constexpr int kThreads = 128;
 // The adjoint's CTAs per SM: 512^2 rays, 96 steps, 256x64x256 cells take
-// 2.21 ms at 5 (96 registers, 16 bytes spilled), 2.32 at 4 (118 registers),
-// 2.27 at 6 and 2.57 at 8 (80 and 64 registers, more spilled).
+// 1362 us at 5 (96 registers) and 1417 us at 6 (80 registers, 112 bytes
+// spilled).
 constexpr int kAdjointCtas = 5;
-constexpr int kMaxCp = 32;   // checkpoints per ray
-constexpr int kMaxSeg = 32;  // steps per checkpoint segment
+// Grid coordinates (cells, cell centres at whole numbers) of a point.
+struct GridPos {
+  float x, y, z;
+};
 
-// Shared-memory words per thread of the adjoint: three transmittances per
-// checkpoint, then a prefix sum and a primary grid value per step of one
-// segment.
-__host__ __device__ constexpr uint32_t adjoint_words(uint32_t n_cp, uint32_t k_cp) {
-  return 3u * n_cp + 2u * k_cp;
+__device__ __forceinline__ GridPos grid_pos(const GridDev& g, float x, float alt, float z) {
+  return {fmaf(x - g.min_x, g.inv_cell_x, -0.5f), fmaf(alt - g.base, g.inv_cell_y, -0.5f),
+          fmaf(z - g.min_z, g.inv_cell_z, -0.5f)};
 }
 
-struct Tri {
-  int x0, y0, z0;
+// The eight corners around a point: the index of its quad in the stored
+// arrays (GridDev::quads, grads) and the weights of the upper corners.  Each
+// coordinate is held to [-2, n]; the arrays hold two layers of zeros before
+// the first cell of every axis and two behind the last, so a point outside
+// reads zeros without a bounds test.  WIDE: arrays too large for floor_bits
+// or a 32-bit index (launch_grid_march).
+template <bool WIDE>
+struct Cell {
+  std::conditional_t<WIDE, size_t, uint32_t> i;  // quad of the lower y row; the upper is g.plane further on
   float wx, wy, wz;
 };
 
-__device__ __forceinline__ Tri grid_coords(const GridDev& g, float x, float alt, float z) {
-  Tri t;
-  const float fx = fmaf(x - g.min_x, g.inv_cell_x, -0.5f);
-  const float fy = fmaf(alt - g.base, g.inv_cell_y, -0.5f);
-  const float fz = fmaf(z - g.min_z, g.inv_cell_z, -0.5f);
-  const float cx = floorf(fminf(fmaxf(fx, -2.0f), (float)g.nx + 1.0f));
-  const float cy = floorf(fminf(fmaxf(fy, -2.0f), (float)g.ny + 1.0f));
-  const float cz = floorf(fminf(fmaxf(fz, -2.0f), (float)g.nz + 1.0f));
-  t.x0 = (int)cx;
-  t.y0 = (int)cy;
-  t.z0 = (int)cz;
-  t.wx = fx - cx;
-  t.wy = fy - cy;
-  t.wz = fz - cz;
-  return t;
-}
-
-// Trilinear fetch without per-corner branches: corner indices clamped into
-// the grid (so every load is in bounds) and the weights of corners outside
-// it zeroed, which gives the same sum as visiting the in-grid corners only;
-// a sample with no corner inside the grid loads nothing.
-// The four (x, z) corners of a y row come as one 16-byte quad
-// (GridDev::quads, zero outside the grid), so x and z need neither clamping
-// nor weight flags: x0 = -1 .. nx-1 and z0 = -1 .. nz-1 have a quad, any
-// other no in-grid corner.  The sum equals the clamped per-corner form term
-// for term (an outside corner adds weight x 0).
-__device__ __forceinline__ float grid_fetch(const GridDev& g, const Tri& t) {
-  const bool xin = (uint32_t)(t.x0 + 1) <= g.nx, zin = (uint32_t)(t.z0 + 1) <= g.nz;
-  const bool y0 = (uint32_t)t.y0 < g.ny, y1 = (uint32_t)(t.y0 + 1) < g.ny;
-  if (!(xin && zin && (y0 || y1))) return 0.0f;
-  const float wx0 = 1.0f - t.wx, wx1 = t.wx;
-  const float wz0 = 1.0f - t.wz, wz1 = t.wz;
-  const float wy[2] = {y0 ? 1.0f - t.wy : 0.0f, y1 ? t.wy : 0.0f};
-  const uint32_t k = (uint32_t)(t.x0 + 1), zk = (uint32_t)(t.z0 + 1), stride = g.nx + 1u;
-  const uint32_t cy[2] = {(uint32_t)min(max(t.y0, 0), (int)g.ny - 1), (uint32_t)min(max(t.y0 + 1, 0), (int)g.ny - 1)};
-  float v = 0.0f;
-#pragma unroll
-  for (int dy = 0; dy < 2; ++dy) {
-    const float4 q = __ldg(g.quads + (cy[dy] * (g.nz + 1u) + zk) * stride + k);
-    v = fmaf(wy[dy] * wz0, fmaf(wx1, q.y, wx0 * q.x), v);
-    v = fmaf(wy[dy] * wz1, fmaf(wx1, q.w, wx0 * q.z), v);
+template <bool WIDE>
+__device__ __forceinline__ Cell<WIDE> grid_cell(const GridDev& g, const GridPos& p) {
+  const float x = fminf(fmaxf(p.x, -2.0f), g.fnx), y = fminf(fmaxf(p.y, -2.0f), g.fny),
+              z = fminf(fmaxf(p.z, -2.0f), g.fnz);
+  Cell<WIDE> c;
+  if constexpr (WIDE) {
+    const float fx = floorf(x), fy = floorf(y), fz = floorf(z);
+    c.i = (size_t)((int64_t)fy + 2) * g.plane + (size_t)((int64_t)fz + 2) * g.row + (size_t)((int64_t)fx + 2);
+    c.wx = x - fx;
+    c.wy = y - fy;
+    c.wz = z - fz;
+  } else {
+    // floor_bits counts from 0x4B400000; g.origin takes that and the two
+    // layers before the first cell off all three axes at once (mod 2^32)
+    const FloorBits fx = floor_bits(x), fy = floor_bits(y), fz = floor_bits(z);
+    c.i = fy.i * (uint32_t)g.plane + fz.i * g.row + (fx.i - g.origin);
+    c.wx = x - fx.f;
+    c.wy = y - fy.f;
+    c.wz = z - fz.f;
   }
-  return v;
+  return c;
 }
 
-// Whether a sample has a corner inside the grid.  One without has grid value
+// Whether a point has a corner inside the grid.  One without has grid value
 // 0 whatever the grid holds, so its value has no gradient either.
-__device__ __forceinline__ bool grid_touches(const GridDev& g, const Tri& t) {
-  return (uint32_t)(t.x0 + 1) <= g.nx && (uint32_t)(t.y0 + 1) <= g.ny && (uint32_t)(t.z0 + 1) <= g.nz;
+__device__ __forceinline__ bool grid_touches(const GridDev& g, const GridPos& p) {
+  return p.x >= -1.0f && p.x < g.fnx && p.y >= -1.0f && p.y < g.fny && p.z >= -1.0f && p.z < g.fnz;
 }
 
-// Adds val x the trilinear weights into the gradient grid: the corners'
-// in-grid flags, clamped indices and weights as in grid_fetch, one atomic add
-// per in-grid corner of non-zero weight (a corner outside the grid has
-// weight zero and is skipped).
-// (into the pair layout GridDev::grad_pairs: one 8-byte vector atomic add
-// per in-grid (y, z) corner pair of non-zero weight; the pair slots outside
-// the grid collect weight that the fold ignores)
-__device__ __forceinline__ void grid_scatter(const GridDev& g, const Tri& t, float val) {
+// Trilinear fetch: the four (x, z) corners of a y row come as one 16-byte
+// quad, blended as two z lanes (FP32x2); a corner outside adds 0.
+template <bool WIDE>
+__device__ __forceinline__ float grid_fetch(const GridDev& g, const Cell<WIDE>& c) {
+  const float wx0 = 1.0f - c.wx, wy0 = 1.0f - c.wy;
+  const float2 x0 = make_float2(wx0, wx0), x1 = make_float2(c.wx, c.wx), wz = make_float2(1.0f - c.wz, c.wz);
+  const float4 a = __ldg(g.quads + c.i), b = __ldg(g.quads + (c.i + (decltype(c.i))g.plane));
+  const float2 ha = fma2(x1, make_float2(a.z, a.w), mul2(x0, make_float2(a.x, a.y)));
+  const float2 hb = fma2(x1, make_float2(b.z, b.w), mul2(x0, make_float2(b.x, b.y)));
+  const float2 v = fma2(mul2(make_float2(c.wy, c.wy), wz), hb, mul2(mul2(make_float2(wy0, wy0), wz), ha));
+  return v.x + v.y;
+}
+
+// Adds val x the trilinear weights into the gradient quads: one 16-byte
+// vector atomic add per y row.  Entries outside the grid collect weight that
+// the fold passes over.
+template <bool WIDE>
+__device__ __forceinline__ void grid_scatter(const GridDev& g, const Cell<WIDE>& c, float val) {
   if (val == 0.0f) return;
-  const bool xin = (uint32_t)(t.x0 + 1) <= g.nx;
-  const bool y0 = (uint32_t)t.y0 < g.ny, y1 = (uint32_t)(t.y0 + 1) < g.ny;
-  const bool z0 = (uint32_t)t.z0 < g.nz, z1 = (uint32_t)(t.z0 + 1) < g.nz;
-  if (!(xin && (y0 || y1) && (z0 || z1))) return;
-  const float wx0 = (1.0f - t.wx) * val, wx1 = t.wx * val;
-  const float wy[2] = {y0 ? 1.0f - t.wy : 0.0f, y1 ? t.wy : 0.0f};
-  const float wz[2] = {z0 ? 1.0f - t.wz : 0.0f, z1 ? t.wz : 0.0f};
-  const uint32_t k = (uint32_t)(t.x0 + 1), stride = g.nx + 1u;
-  const uint32_t cy[2] = {(uint32_t)min(max(t.y0, 0), (int)g.ny - 1), (uint32_t)min(max(t.y0 + 1, 0), (int)g.ny - 1)};
-  const uint32_t cz[2] = {(uint32_t)min(max(t.z0, 0), (int)g.nz - 1), (uint32_t)min(max(t.z0 + 1, 0), (int)g.nz - 1)};
+  const float z1 = c.wz * val, z0 = (1.0f - c.wz) * val;
+  const float x1 = c.wx, x0 = 1.0f - c.wx;
+  const float4 q = make_float4(x0 * z0, x0 * z1, x1 * z0, x1 * z1);
+  const float wy[2] = {1.0f - c.wy, c.wy};
 #pragma unroll
   for (int dy = 0; dy < 2; ++dy)
-#pragma unroll
-    for (int dz = 0; dz < 2; ++dz) {
-      const float wyz = wy[dy] * wz[dz];
-      if (wyz != 0.0f)
-        atomicAdd(g.grad_pairs + (cy[dy] * g.nz + cz[dz]) * stride + k, make_float2(wyz * wx0, wyz * wx1));
-    }
+    if (wy[dy] != 0.0f)
+      atomicAdd(g.grads + (c.i + (decltype(c.i))(dy ? g.plane : 0)),
+                make_float4(wy[dy] * q.x, wy[dy] * q.y, wy[dy] * q.z, wy[dy] * q.w));
 }
 
-// Light march geometry (cloud_march.wgsl:543-578).
-struct LightGeo {
-  float r0, cv, delta;
+// A point of the march: position, altitude and local up.
+struct Sample {
+  float x, y, z, alt, ux, uy, uz;
 };
 
-__device__ __forceinline__ LightGeo light_geo(const MarchUniforms& u, const LayerConst& L, float alt,
-                                              float ux, float uy, float uz) {
+// Light march of one sample (cloud_march.wgsl:543-578) in grid coordinates:
+// x and z are affine along the sun ray, and for light paths up to 20 km the
+// altitude is the cubic of march_fast_body.cuh's LightRay (truncation below
+// 1e-4 m); longer ones take the altitude of each tap from the geometry.
+struct LightGeo {
+  float x, z, kx, kz;    // x + kx t, z + kz t
+  float c0, c1, c2, c3;  // y = c0 + t (c1 + t (c2 + t c3))
+  float delta;           // metres per tap
+  bool poly;
+};
+
+__device__ __forceinline__ LightGeo light_geo(const MarchUniforms& u, const GridDev& g, const LayerConst& L,
+                                              const GridPos& p, const Sample& q) {
   LightGeo lg;
-  lg.r0 = u.planet_r + alt;
-  lg.cv = fmaf(ux, u.sun[0], fmaf(uy, u.sun[1], uz * u.sun[2]));
-  lg.delta = __fdividef(fmaxf((L.top_m - alt) * u.inv_cos_sun, 1.0f), (float)u.light_steps);
+  const float r0 = u.planet_r + q.alt;
+  const float cv = fmaf(q.ux, u.sun[0], fmaf(q.uy, u.sun[1], q.uz * u.sun[2]));
+  const float dist = fmaxf((L.top_m - q.alt) * u.inv_cos_sun, 1.0f);
+  lg.delta = __fdividef(dist, (float)u.light_steps);
+  lg.poly = dist <= 20000.0f;
+  const float s2 = fmaf(-cv, cv, 1.0f) * __fdividef(0.5f, r0);
+  lg.x = p.x;
+  lg.z = p.z;
+  lg.kx = u.sun[0] * g.inv_cell_x;
+  lg.kz = u.sun[2] * g.inv_cell_z;
+  lg.c0 = p.y;
+  lg.c1 = cv * g.inv_cell_y;
+  lg.c2 = s2 * g.inv_cell_y;
+  lg.c3 = -cv * __fdividef(s2, r0) * g.inv_cell_y;
   return lg;
 }
 
-__device__ __forceinline__ Tri light_tap(const MarchUniforms& u, const GridDev& g, const LightGeo& lg,
-                                         float px3, float py3, float pz3, float alt, uint32_t j) {
-  const float t = ((float)j + 0.5f) * lg.delta;
-  const float qx = fmaf(u.sun[0], t, px3), qy = fmaf(u.sun[1], t, py3), qz = fmaf(u.sun[2], t, pz3);
-  return grid_coords(g, qx, alt_from(u, qx, qy, qz, lg.r0, lg.cv, alt, t), qz);
+__device__ __forceinline__ GridPos light_pos(const LightGeo& lg, float t) {
+  return {fmaf(lg.kx, t, lg.x), fmaf(t, fmaf(t, fmaf(t, lg.c3, lg.c2), lg.c1), lg.c0), fmaf(lg.kz, t, lg.z)};
+}
+// The tap of a path over 20 km.
+__device__ __forceinline__ GridPos light_pos_far(const MarchUniforms& u, const GridDev& g, const LightGeo& lg,
+                                                 const Sample& p, float t) {
+  const float qx = fmaf(u.sun[0], t, p.x), qy = fmaf(u.sun[1], t, p.y), qz = fmaf(u.sun[2], t, p.z);
+  const float cv = fmaf(p.ux, u.sun[0], fmaf(p.uy, u.sun[1], p.uz * u.sun[2]));
+  const float alt = alt_from(u, qx, qy, qz, u.planet_r + p.alt, cv, p.alt, t);
+  return {fmaf(lg.kx, t, lg.x), fmaf(alt - g.base, g.inv_cell_y, -0.5f), fmaf(lg.kz, t, lg.z)};
 }
 
-__device__ __forceinline__ float light_sum(const MarchUniforms& u, const GridDev& g, const LightGeo& lg,
-                                           float px3, float py3, float pz3, float alt) {
+template <bool WIDE>
+__device__ __forceinline__ float light_sum(const MarchUniforms& u, const GridDev& g, const LightGeo& lg, const Sample& p) {
   float s = 0.0f;
-  for (uint32_t j = 0; j < u.light_steps; ++j) s += grid_fetch(g, light_tap(u, g, lg, px3, py3, pz3, alt, j));
+  if (lg.poly) {
+    // the tap index as a float, in groups of three
+    const float n = (float)u.light_steps;
+    float j = 0.5f;
+#pragma unroll 1
+    for (; j + 2.0f < n; j += 3.0f) {
+      float v[3];
+#pragma unroll
+      for (int k = 0; k < 3; ++k) v[k] = grid_fetch<WIDE>(g, grid_cell<WIDE>(g, light_pos(lg, (j + (float)k) * lg.delta)));
+      s = ((s + v[0]) + v[1]) + v[2];
+    }
+#pragma unroll 1
+    for (; j < n; j += 1.0f) s += grid_fetch<WIDE>(g, grid_cell<WIDE>(g, light_pos(lg, j * lg.delta)));
+  } else {
+#pragma unroll 1
+    for (uint32_t j = 0; j < u.light_steps; ++j)
+      s += grid_fetch<WIDE>(g, grid_cell<WIDE>(g, light_pos_far(u, g, lg, p, ((float)j + 0.5f) * lg.delta)));
+  }
   return s * lg.delta;
+}
+
+// d loss / d (light sum) of every tap into the gradient.
+template <bool WIDE>
+__device__ __forceinline__ void light_scatter(const MarchUniforms& u, const GridDev& g, const LightGeo& lg,
+                                              const Sample& p, float val) {
+#pragma unroll 1
+  for (uint32_t j = 0; j < u.light_steps; ++j) {
+    const float t = ((float)j + 0.5f) * lg.delta;
+    const GridPos q = lg.poly ? light_pos(lg, t) : light_pos_far(u, g, lg, p, t);
+    if (grid_touches(g, q)) grid_scatter<WIDE>(g, grid_cell<WIDE>(g, q), val);
+  }
 }
 
 // (1 - e^-x) / x with e = e^-x.
@@ -181,9 +226,8 @@ struct Light {
 };
 
 __device__ __forceinline__ void lighting(const MarchUniforms& u, const LayerConst& L, const float* coef,
-                                         bool cb, float cos_theta, float fwd_gain, float px3, float pz3,
-                                         float alt, float ux, float uy, float uz, Light& l) {
-  const float h = clamp01((alt - L.base_m) * L.inv_thickness);
+                                         bool cb, float cos_theta, float fwd_gain, const Sample& p, Light& l) {
+  const float h = clamp01((p.alt - L.base_m) * L.inv_thickness);
   if (cb) {
     const float mt = smoothstepf(0.60f, 0.85f, h);
     const PhaseConst pc = phase_consts_from_d(mixf(L.droplet_um, 50.0f, mt), u.droplet_bias);
@@ -195,14 +239,14 @@ __device__ __forceinline__ void lighting(const MarchUniforms& u, const LayerCons
     for (int n = 0; n < kMaxOct; ++n) l.cf[n] = coef[n];
   }
   float3 ts, sky;
-  lut_lookups(u, alt, ux, uy, uz, ts, sky);
+  lut_lookups(u, p.alt, p.ux, p.uy, p.uz, ts, sky);
   l.sun[0] = u.sun_illum[0] * ts.x;
   l.sun[1] = u.sun_illum[1] * ts.y;
   l.sun[2] = u.sun_illum[2] * ts.z;
   const float ag = mixf(0.3f, 1.0f, h) * u.ambient;
   float lr = 0.0f, lg = 0.0f, lb = 0.0f;
   if (u.lightning_radius > 0.0f) {
-    const float ddx = px3 - u.lightning_origin_x, ddz = pz3 - u.lightning_origin_z;
+    const float ddx = p.x - u.lightning_origin_x, ddz = p.z - u.lightning_origin_z;
     const float fo = clamp01(1.0f - sqrtf(ddx * ddx + ddz * ddz) / u.lightning_radius);
     const float wgt = fo * fo * (3.0f - 2.0f * fo);
     lr = u.lightning_rgb[0] * wgt;
@@ -242,12 +286,9 @@ __device__ __forceinline__ float source(const MarchUniforms& u, const Light& l, 
   return fmaf(S, E, l.amb[c]);
 }
 
-// `sm` is this thread's column of the adjoint's shared memory (stride
-// kThreads words); unused by the forward form.
-template <bool ADJ>
+template <bool ADJ, bool WIDE>
 __device__ __forceinline__ void grid_pixel(const MarchUniforms& u, const ViewDev& v, const GridDev& g,
-                                           uint32_t px, uint32_t py, float* sm, float& loss_out,
-                                           float& dk_out) {
+                                           uint32_t px, uint32_t py, float& loss_out, float& dk_out) {
   RaySetup rs;
   setup_ray(u, v, px, py, rs);
   const LayerConst& L = u.layers[0];
@@ -287,49 +328,60 @@ __device__ __forceinline__ void grid_pixel(const MarchUniforms& u, const ViewDev
   const float t0 = rs.t0[0], t1 = rs.t1[0];
   const bool hit = (rs.hit_mask & 1u) && t1 > t0;
   const float step = hit ? __fdividef(t1 - t0, (float)u.cloud_steps) : 0.0f;
-  const uint32_t kcp = g.k_cp;
   uint32_t n_exec = 0;
-  // shared-memory slots: checkpoint transmittances, then the segment's
-  // prefix sums, primary grid values and light sums
-  float* const s_cp = sm;
-  float* const s_pre = sm + 3u * ((u.cloud_steps + kcp - 1u) / kcp) * kThreads;
-  float* const s_gv = s_pre + kcp * kThreads;
+  double pre = 0.0;  // adjoint: sum of the grid values of the executed steps
   // an infinity or NaN somewhere in the grid reaches L through the light sum
   // of an empty sample (0 x inf), so such a grid has every sample lit
   const bool every = __ldg(g.nonfinite) != 0u;
 
-  auto position = [&](uint32_t s, float& px3, float& py3, float& pz3, float& alt, float& ux, float& uy,
-                      float& uz) {
+  auto position = [&](uint32_t s) {
+    Sample p;
     const float t = fmaf((float)s + jitter, step, t0);
-    px3 = fmaf(dx, t, cx);
-    py3 = fmaf(dy, t, cy);
-    pz3 = fmaf(dz, t, cz);
-    alt = alt_from(u, px3, py3, pz3, ray_r0, ray_cv, ray_h0, t);
-    const float inv_r = __frcp_rn(u.planet_r + alt);
-    ux = px3 * inv_r;
-    uy = (py3 + u.planet_r) * inv_r;
-    uz = pz3 * inv_r;
+    p.x = fmaf(dx, t, cx);
+    p.y = fmaf(dy, t, cy);
+    p.z = fmaf(dz, t, cz);
+    p.alt = alt_from(u, p.x, p.y, p.z, ray_r0, ray_cv, ray_h0, t);
+    const float inv_r = __frcp_rn(u.planet_r + p.alt);
+    p.ux = p.x * inv_r;
+    p.uy = (p.y + u.planet_r) * inv_r;
+    p.uz = p.z * inv_r;
+    return p;
   };
 
   if (hit) {
-    for (uint32_t s = 0; s < u.cloud_steps; ++s) {
-      if constexpr (ADJ) {
-        if (s % kcp == 0) {
-          const uint32_t c0 = 3u * (s / kcp) * kThreads;
-          s_cp[c0] = T[0];
-          s_cp[c0 + kThreads] = T[1];
-          s_cp[c0 + 2u * kThreads] = T[2];
-        }
+    // The grid values of kAhead steps are fetched together, so that an empty
+    // stretch waits for one fetch latency per group: forward 512^2 view 295 us
+    // one by one, 258 / 261 / 238 / 248 us in groups of 2 / 4 / 6 / 8; adjoint
+    // 1362 us one by one, 1320 / 1332 / 1345 us in groups of 2 / 4 / 6.
+    constexpr uint32_t kAhead = ADJ ? 2u : 6u;
+    n_exec = u.cloud_steps;
+    for (uint32_t s0 = 0; s0 < u.cloud_steps; s0 += kAhead) {
+      float gvs[kAhead];
+      bool any = every;
+#pragma unroll
+      for (uint32_t k = 0; k < kAhead; ++k) {
+        const Sample p = position(s0 + k);
+        const float gv = grid_fetch<WIDE>(g, grid_cell<WIDE>(g, grid_pos(g, p.x, p.alt, p.z)));
+        gvs[k] = s0 + k < u.cloud_steps ? gv : 0.0f;
+        any = any || gvs[k] != 0.0f;
       }
-      float px3, py3, pz3, alt, ux, uy, uz;
-      position(s, px3, py3, pz3, alt, ux, uy, uz);
-      const float gv = grid_fetch(g, grid_coords(g, px3, alt, pz3));
-      if (gv != 0.0f || every) {
-        const LightGeo lg = light_geo(u, L, alt, ux, uy, uz);
-        const float gl = light_sum(u, g, lg, px3, py3, pz3, alt);
+      if (!any) continue;
+      bool done = false;
+#pragma unroll 1
+      for (uint32_t k = 0; k < kAhead; ++k) {
+        const uint32_t s = s0 + k;
+        float gv = gvs[0];
+#pragma unroll
+        for (uint32_t j = 1; j < kAhead; ++j) gv = k == j ? gvs[j] : gv;
+        if (s >= u.cloud_steps || (gv == 0.0f && !every)) continue;
+        const Sample p = position(s);
+        const GridPos gp = grid_pos(g, p.x, p.alt, p.z);
+        if constexpr (ADJ) pre += (double)gv;
+        const LightGeo lg = light_geo(u, g, L, gp, p);
+        const float gl = light_sum<WIDE>(u, g, lg, p);
         const float rho = g.k * gv, od = g.k * gl;
         Light l;
-        lighting(u, L, coef, cb, cos_theta, fwd_gain, px3, pz3, alt, ux, uy, uz, l);
+        lighting(u, L, coef, cb, cos_theta, fwd_gain, p, l);
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
           const float X = source<false>(u, l, st[c], c, od, nullptr);
@@ -338,9 +390,13 @@ __device__ __forceinline__ void grid_pixel(const MarchUniforms& u, const ViewDev
           Lc[c] = fmaf(T[c], rho * ss[c] * X * step * phi_of(x, e), Lc[c]);
           T[c] *= e;
         }
+        if (fmaxf(T[0], fmaxf(T[1], T[2])) < g.exit_t) {
+          n_exec = s + 1u;
+          done = true;
+          break;
+        }
       }
-      n_exec = s + 1;
-      if (fmaxf(T[0], fmaxf(T[1], T[2])) < g.exit_t) break;
+      if (done) break;
     }
   }
 
@@ -372,57 +428,61 @@ __device__ __forceinline__ void grid_pixel(const MarchUniforms& u, const ViewDev
   float dk = 0.0f;
   if (n_exec > 0) {
     const float kstep = g.k * step;
-    for (int seg = (int)((n_exec - 1) / kcp); seg >= 0; --seg) {
-      const uint32_t s0 = (uint32_t)seg * kcp;
-      const uint32_t s1 = min(s0 + kcp, n_exec);
-      float pre = 0.0f;
-      for (uint32_t s = s0; s < s1; ++s) {  // refetch the segment's grid values
-        float px3, py3, pz3, alt, ux, uy, uz;
-        position(s, px3, py3, pz3, alt, ux, uy, uz);
-        const float gv = grid_fetch(g, grid_coords(g, px3, alt, pz3));
-        const uint32_t b = (s - s0) * kThreads;
-        s_pre[b] = pre;
-        s_gv[b] = gv;
-        pre += gv;
+    float bT[3] = {T[0], T[1], T[2]};  // transmittance before the step
+    for (uint32_t s = n_exec; s-- > 0u;) {
+      const Sample p = position(s);
+      const GridPos gp = grid_pos(g, p.x, p.alt, p.z);
+      const Cell<WIDE> cell = grid_cell<WIDE>(g, gp);
+      // outside the grid: no gradient, and lam passes unchanged
+      const bool in = grid_touches(g, gp);
+      if (!in && !every) continue;
+      const float gv = grid_fetch<WIDE>(g, cell);
+      if (gv != 0.0f || every) {
+        pre -= (double)gv;
+        const float p_od = kstep * (float)pre;  // optical depth per unit sigma_t before the step
+#pragma unroll
+        for (int c = 0; c < 3; ++c) bT[c] = __expf(-st[c] * p_od);
       }
-      const uint32_t c0 = 3u * (uint32_t)seg * kThreads;
-      const float cp3[3] = {s_cp[c0], s_cp[c0 + kThreads], s_cp[c0 + 2u * kThreads]};
-      for (uint32_t s = s1; s-- > s0;) {  // reverse
-        const uint32_t b = (s - s0) * kThreads;
-        float px3, py3, pz3, alt, ux, uy, uz;
-        position(s, px3, py3, pz3, alt, ux, uy, uz);
-        const Tri tri = grid_coords(g, px3, alt, pz3);
-        // outside the grid: no gradient, and lam passes unchanged
-        if (!grid_touches(g, tri) && !every) continue;
-        const LightGeo lg = light_geo(u, L, alt, ux, uy, uz);
-        const float gv = s_gv[b], gl = light_sum(u, g, lg, px3, py3, pz3, alt);
-        const float p_od = kstep * s_pre[b];  // optical depth per unit sigma_t since the checkpoint
-        const float bT[3] = {cp3[0] * __expf(-st[0] * p_od), cp3[1] * __expf(-st[1] * p_od),
-                             cp3[2] * __expf(-st[2] * p_od)};
-        const float rho = g.k * gv, od = g.k * gl;
-        Light l;
-        lighting(u, L, coef, cb, cos_theta, fwd_gain, px3, pz3, alt, ux, uy, uz, l);
-        float drho = 0.0f, dod = 0.0f;
+      const LightGeo lg = light_geo(u, g, L, gp, p);
+      const float gl = light_sum<WIDE>(u, g, lg, p);
+      const float rho = g.k * gv, od = g.k * gl;
+      Light l;
+      lighting(u, L, coef, cb, cos_theta, fwd_gain, p, l);
+      float drho = 0.0f, dod = 0.0f;
+      float s_lit = 0.0f;
+#pragma unroll
+      for (int n = 0; n < kMaxOct; ++n) s_lit += l.cf[n];
+      if (gv == 0.0f && !every) {
+        // rho = 0: e = 1, the step adds nothing to L and lam stays; only
+        // the derivative in rho is left
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-          float dX;
-          const float X = source<true>(u, l, st[c], c, od, &dX);
-          const float x = rho * st[c] * step;
-          const float e = __expf(-x), ph = phi_of(x, e);
-          const float s_int = rho * ss[c] * X * step * ph;
-          const float gT = gI[c] * bT[c];
-          drho = fmaf(gT, ss[c] * X * step * e, drho);
-          drho = fmaf(lam[c] * bT[c], -st[c] * step * e, drho);
-          dod = fmaf(gT * rho * ss[c] * step * ph, dX, dod);
-          lam[c] = fmaf(lam[c], e, gI[c] * s_int);
+          // nothing toward the sun either: every exponential is 1
+          const float X = od == 0.0f ? fmaf(s_lit * l.sun[c], 1.0f - u.powder, l.amb[c])
+                                     : source<false>(u, l, st[c], c, od, nullptr);
+          drho = fmaf(gI[c] * bT[c], ss[c] * X * step, drho);
+          drho = fmaf(lam[c] * bT[c], -st[c] * step, drho);
         }
-        grid_scatter(g, tri, g.k * drho);
-        const float vl = g.k * lg.delta * dod;
-        if (vl != 0.0f)
-          for (uint32_t j = 0; j < u.light_steps; ++j)
-            grid_scatter(g, light_tap(u, g, lg, px3, py3, pz3, alt, j), vl);
-        dk = fmaf(gv, drho, fmaf(gl, dod, dk));
+        grid_scatter<WIDE>(g, cell, g.k * drho);
+        continue;
       }
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        float dX;
+        const float X = source<true>(u, l, st[c], c, od, &dX);
+        const float x = rho * st[c] * step;
+        const float e = __expf(-x), ph = phi_of(x, e);
+        const float s_int = rho * ss[c] * X * step * ph;
+        const float gT = gI[c] * bT[c];
+        drho = fmaf(gT, ss[c] * X * step * e, drho);
+        drho = fmaf(lam[c] * bT[c], -st[c] * step * e, drho);
+        dod = fmaf(gT * rho * ss[c] * step * ph, dX, dod);
+        lam[c] = fmaf(lam[c], e, gI[c] * s_int);
+      }
+      if (in) grid_scatter<WIDE>(g, cell, g.k * drho);
+      const float vl = g.k * lg.delta * dod;
+      if (vl != 0.0f) light_scatter<WIDE>(u, g, lg, p, vl);
+      dk = fmaf(gv, drho, fmaf(gl, dod, dk));
     }
   }
   dk_out = dk;
@@ -437,21 +497,23 @@ __device__ __forceinline__ double warp_sum(double x) {
 
 // MINB: CTAs per SM the register allocation is bounded for (0: unbounded).
 //
-// Both forms are instruction bound (the grid and its gradient stay in L2).
-// Lighting only the samples the grid is not empty at takes the forward march
-// of 512^2 rays, 96 + 6 steps, 256x64x256 cells at 13 % fill from 1.20 to
-// 0.34 ms (983 M to 181 M warp instructions); one light march per sample
-// instead of two takes the adjoint from 3.76 to 2.21 ms (2366 M to 1557 M).
-template <bool ADJ, int MINB>
+// Both forms are bound by instructions and by fetch latency (the grid and its
+// gradient stay in L2).  512^2 rays, 96 + 6 steps, 256x64x256 cells at 13 %
+// fill: lighting only the samples the grid is not empty at took the forward
+// march from 1204 to 338 us (983 M to 181 M warp instructions) and one light
+// march per sample instead of two the adjoint from 3759 to 2211 us (2366 M to
+// 1557 M); zero-padded arrays without bounds tests, FP32x2 blends and cubic
+// tap heights took them to 295 and 1886 us, and the steps named above to 238
+// and 1320 us (801 M).
+template <bool ADJ, int MINB, bool WIDE>
 __global__ void __launch_bounds__(kThreads, MINB) k_grid_march(const __grid_constant__ MarchUniforms u,
                                                                const __grid_constant__ ViewDev v,
                                                                const __grid_constant__ GridDev g) {
-  extern __shared__ float s_adj[];
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   const uint32_t px = blockIdx.x * kTileW + (warp & 1u) * 8u + (lane & 7u);
   const uint32_t py = blockIdx.y * kTileH + (warp >> 1) * 4u + (lane >> 3);
   float loss = 0.0f, dk = 0.0f;
-  if (px < v.width && py < v.height) grid_pixel<ADJ>(u, v, g, px, py, s_adj + threadIdx.x, loss, dk);
+  if (px < v.width && py < v.height) grid_pixel<ADJ, WIDE>(u, v, g, px, py, loss, dk);
   if (!ADJ) return;
   __shared__ double s_red[2][kThreads / 32];
   const double ls = warp_sum((double)loss), ks = warp_sum((double)dk);
@@ -472,48 +534,43 @@ __global__ void __launch_bounds__(kThreads, MINB) k_grid_march(const __grid_cons
   }
 }
 
-cudaError_t launch_adjoint(const MarchUniforms& u, const ViewDev& v, const GridDev& g, dim3 grid,
-                           size_t smem, cudaStream_t s) {
-  if (smem > 48u * 1024u) {
-    const cudaError_t e = cudaFuncSetAttribute(k_grid_march<true, kAdjointCtas>,
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-  }
-  k_grid_march<true, kAdjointCtas><<<grid, kThreads, smem, s>>>(u, v, g);
-  return cudaGetLastError();
-}
-
-// One warp per (y, zk) row of quads, so no index is divided per quad.  Sets
+// One warp per (yi, zi) row of quads, so no index is divided per quad.  Sets
 // *nonfinite when a value is an infinity or NaN.
 __global__ void __launch_bounds__(256) k_grid_quads(const float* __restrict__ v, float4* __restrict__ q,
                                                     uint32_t nx, uint32_t ny, uint32_t nz,
                                                     uint32_t* __restrict__ nonfinite) {
-  const uint32_t lane = threadIdx.x & 31u, sz = nz + 1u, rows = ny * sz, warps = gridDim.x * (blockDim.x >> 5);
+  const uint32_t lane = threadIdx.x & 31u, sz = nz + 3u, sx = nx + 3u;
+  const uint64_t rows = (uint64_t)(ny + 4u) * sz, warps = (uint64_t)gridDim.x * (blockDim.x >> 5);
   bool bad = false;
-  for (uint32_t row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); row < rows; row += warps) {
-    const uint32_t y = row / sz, zk = row - y * sz;
-    const float* const a = v + ((size_t)y * nz + zk) * nx - nx;  // row zk - 1 of the grid, read if zk > 0
-    const bool lo = zk > 0u, hi = zk < nz;
-    float4* const out = q + (size_t)row * (nx + 1u);
-    for (uint32_t xk = lane; xk <= nx; xk += 32u) {
-      const bool l = xk > 0u, r = xk < nx;
-      const float4 t = make_float4(lo && l ? __ldg(a + xk - 1u) : 0.0f, lo && r ? __ldg(a + xk) : 0.0f,
-                                   hi && l ? __ldg(a + nx + xk - 1u) : 0.0f, hi && r ? __ldg(a + nx + xk) : 0.0f);
-      bad = bad || !isfinite(t.y) || !isfinite(t.w);  // every cell is some quad's right column
-      out[xk] = t;
+  for (uint64_t row = (uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); row < rows; row += warps) {
+    const uint32_t yi = (uint32_t)(row / sz), zi = (uint32_t)(row - (uint64_t)yi * sz);
+    const bool in = yi >= 2u && yi - 2u < ny;
+    const bool lo = in && zi >= 2u && zi - 2u < nz, hi = in && zi >= 1u && zi - 1u < nz;  // z = zi - 2 and zi - 1
+    const float* const a = v + ((size_t)(in ? yi - 2u : 0u) * nz + (lo ? zi - 2u : 0u)) * nx;
+    const float* const b = v + ((size_t)(in ? yi - 2u : 0u) * nz + (hi ? zi - 1u : 0u)) * nx;
+    float4* const out = q + (size_t)row * sx;
+    for (uint32_t xi = lane; xi < sx; xi += 32u) {
+      const bool l = xi >= 2u && xi - 2u < nx, r = xi >= 1u && xi - 1u < nx;  // x = xi - 2 and xi - 1
+      const float4 t = make_float4(lo && l ? __ldg(a + xi - 2u) : 0.0f, hi && l ? __ldg(b + xi - 2u) : 0.0f,
+                                   lo && r ? __ldg(a + xi - 1u) : 0.0f, hi && r ? __ldg(b + xi - 1u) : 0.0f);
+      bad = bad || !isfinite(t.w);  // every cell is some quad's upper right corner
+      out[xi] = t;
     }
   }
   if (bad) *nonfinite = 1u;
 }
 
-// grad += the two pair entries of each cell, one warp per (y, z) row.
-__global__ void __launch_bounds__(256) k_grid_fold(const float2* __restrict__ gp, float* __restrict__ grad,
-                                                   uint32_t nx, uint32_t rows) {
-  const uint32_t lane = threadIdx.x & 31u, warps = gridDim.x * (blockDim.x >> 5);
+// grad += the four quad entries of each cell, one warp per (y, z) row.
+__global__ void __launch_bounds__(256) k_grid_fold(const float4* __restrict__ gq, float* __restrict__ grad,
+                                                   uint32_t nx, uint32_t ny, uint32_t nz) {
+  const uint32_t lane = threadIdx.x & 31u, warps = gridDim.x * (blockDim.x >> 5), rows = ny * nz, sx = nx + 3u;
   for (uint32_t r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); r < rows; r += warps) {
-    const float2* const row = gp + (size_t)r * (nx + 1u);
+    const uint32_t y = r / nz, z = r - y * nz;
+    const float4* const up = gq + ((size_t)(y + 2u) * (nz + 3u) + z + 2u) * sx;  // quads whose lower z is z
+    const float4* const dn = up - sx;
     float* const out = grad + (size_t)r * nx;
-    for (uint32_t x = lane; x < nx; x += 32u) out[x] += __ldg(row + x + 1u).x + __ldg(row + x).y;
+    for (uint32_t x = lane; x < nx; x += 32u)
+      out[x] += (__ldg(up + x + 2u).x + __ldg(up + x + 1u).z) + (__ldg(dn + x + 2u).y + __ldg(dn + x + 1u).w);
   }
 }
 
@@ -526,26 +583,27 @@ int launch_grid_quads(const float* values, float4* quads, uint32_t* nonfinite, u
   return cudaGetLastError() == cudaSuccess ? PSC_OK : PSC_ERR_CUDA;
 }
 
-int launch_grid_fold(const float2* grad_pairs, float* grad, uint32_t nx, uint32_t rows, cudaStream_t s) {
-  k_grid_fold<<<148u * 8u, 256, 0, s>>>(grad_pairs, grad, nx, rows);
+int launch_grid_fold(const float4* grads, float* grad, uint32_t nx, uint32_t ny, uint32_t nz, cudaStream_t s) {
+  k_grid_fold<<<148u * 8u, 256, 0, s>>>(grads, grad, nx, ny, nz);
   return cudaGetLastError() == cudaSuccess ? PSC_OK : PSC_ERR_CUDA;
 }
 
 int launch_grid_march(const MarchUniforms& u, const ViewDev& v, const GridDev& g, bool adjoint,
                       cudaStream_t s) {
-  if (!g.quads || (adjoint && !g.grad_pairs)) return PSC_ERR_INVALID_ARGUMENT;
+  if (!g.quads || (adjoint && !g.grads)) return PSC_ERR_INVALID_ARGUMENT;
   if (u.octaves == 0 || u.octaves > (uint32_t)kMaxOct) return PSC_ERR_UNSUPPORTED;
-  if (adjoint && (g.k_cp == 0 || g.k_cp > (uint32_t)kMaxSeg ||
-                  (u.cloud_steps + g.k_cp - 1) / g.k_cp > (uint32_t)kMaxCp))
-    return PSC_ERR_INVALID_ARGUMENT;
   const dim3 grid((v.width + kTileW - 1) / kTileW, (v.height + kTileH - 1) / kTileH);
-  if (adjoint) {
-    // at most 3 x 32 + 2 x 32 words per thread (80 KiB per CTA)
-    const uint32_t n_cp = (u.cloud_steps + g.k_cp - 1) / g.k_cp;
-    const size_t smem = (size_t)adjoint_words(n_cp, g.k_cp) * kThreads * sizeof(float);
-    return launch_adjoint(u, v, g, grid, smem, s) == cudaSuccess ? PSC_OK : PSC_ERR_CUDA;
-  }
-  k_grid_march<false, 0><<<grid, kThreads, 0, s>>>(u, v, g);
+  // floor_bits counts cells exactly up to 2^22; the narrow kernels index in 32 bits
+  const bool wide = g.nx >= (1u << 21) || g.ny >= (1u << 21) || g.nz >= (1u << 21) ||
+                    g.plane * (g.ny + 4ull) >= (1ull << 31);
+  if (adjoint && wide)
+    k_grid_march<true, kAdjointCtas, true><<<grid, kThreads, 0, s>>>(u, v, g);
+  else if (adjoint)
+    k_grid_march<true, kAdjointCtas, false><<<grid, kThreads, 0, s>>>(u, v, g);
+  else if (wide)
+    k_grid_march<false, 0, true><<<grid, kThreads, 0, s>>>(u, v, g);
+  else
+    k_grid_march<false, 0, false><<<grid, kThreads, 0, s>>>(u, v, g);
   return cudaGetLastError() == cudaSuccess ? PSC_OK : PSC_ERR_CUDA;
 }
 

@@ -98,11 +98,11 @@ struct psc_ctx {
   std::vector<cudaTextureObject_t> batch_sky_tex;  // per-view sky-view LUTs through the texture unit
   float4* d_bap = nullptr;              // per-view aerial-perspective LUTs
   // voxel-grid form: the grid values as corner quads and the adjoint's
-  // gradient as x pairs (GridDev::quads / grad_pairs), grown to the largest
-  // grid seen; GridDev::nonfinite lies behind the quads
+  // gradient in the same form (GridDev::quads / grads), each grown to the
+  // largest grid seen; GridDev::nonfinite lies behind the quads
   float4* d_grid_quads = nullptr;
-  float2* d_grad_pairs = nullptr;
-  size_t grid_pairs_cap = 0;  // entries of the quad array (the pair array holds as many)
+  float4* d_grid_grads = nullptr;
+  size_t grid_quads_cap = 0, grid_grads_cap = 0;  // entries
   uint32_t* d_btiles = nullptr;
   uint32_t* d_bcounter = nullptr;
   psc::MarchUniforms* h_bu = nullptr;   // pinned staging

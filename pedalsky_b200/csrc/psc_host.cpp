@@ -1545,7 +1545,7 @@ int psc_destroy(psc_ctx* c) {
   dfree(c->d_rt_depth);
   dfree(c->d_check);
   dfree(c->d_grid_quads);
-  dfree(c->d_grad_pairs);
+  dfree(c->d_grid_grads);
   for (auto& tv : c->taa) free_taa_view(tv);
   dfree(c->d_blue);
   dfree(c->d_weather);
@@ -2454,7 +2454,16 @@ int prepare_grid(psc_ctx* c, const PscDensityGrid* g, const PscView* v, bool adj
   gd.nx = g->nx;
   gd.ny = g->ny;
   gd.nz = g->nz;
-  gd.k_cp = g->checkpoint_every;
+  auto not_above = [](uint32_t n) {  // n as a float, rounded down: a bound of cell indices
+    const float f = (float)n;
+    return (double)f > (double)n ? std::nextafter(f, 0.0f) : f;
+  };
+  gd.fnx = not_above(g->nx);
+  gd.fny = not_above(g->ny);
+  gd.fnz = not_above(g->nz);
+  gd.row = g->nx + 3u;
+  gd.plane = (uint64_t)(g->nz + 3u) * gd.row;
+  gd.origin = (uint32_t)((gd.plane + gd.row + 1u) * 0x4B3FFFFEull);  // 0x4B400000 - 2 per axis
   gd.min_x = g->min_x_m;
   gd.min_z = g->min_z_m;
   gd.base = L.base_m;
@@ -2469,26 +2478,25 @@ int prepare_grid(psc_ctx* c, const PscDensityGrid* g, const PscView* v, bool adj
 }
 
 // The grid values as (x, z) corner quads (GridDev::quads) on `s`, and for the
-// adjoint a zeroed gradient in x pairs (GridDev::grad_pairs).
+// adjoint a zeroed gradient of the same form (GridDev::grads).
 int stage_grid_layout(psc_ctx* c, psc::GridDev& gd, bool adjoint, cudaStream_t s) {
-  const size_t nq = (size_t)gd.ny * (gd.nz + 1u) * (gd.nx + 1u);  // quads
-  const size_t np = (size_t)gd.ny * gd.nz * (gd.nx + 1u);         // gradient pairs
-  if (c->grid_pairs_cap < nq) {
+  const size_t nq = (size_t)gd.plane * (gd.ny + 4u);
+  if (c->grid_quads_cap < nq) {
     dfree(c->d_grid_quads);
-    dfree(c->d_grad_pairs);
-    c->grid_pairs_cap = 0;
+    c->grid_quads_cap = 0;
     PSC_CUDA(cudaMalloc(&c->d_grid_quads, (nq + 1u) * sizeof(float4)), "cudaMalloc grid quads");  // + the flag
-    PSC_CUDA(cudaMalloc(&c->d_grad_pairs, nq * sizeof(float2)), "cudaMalloc gradient pairs");
-    c->grid_pairs_cap = nq;
+    c->grid_quads_cap = nq;
   }
-  uint32_t* const nonfinite = reinterpret_cast<uint32_t*>(c->d_grid_quads + c->grid_pairs_cap);
+  uint32_t* const nonfinite = reinterpret_cast<uint32_t*>(c->d_grid_quads + c->grid_quads_cap);
   if (psc::launch_grid_quads(gd.values, c->d_grid_quads, nonfinite, gd.nx, gd.ny, gd.nz, s))
     return fail(PSC_ERR_CUDA, "grid quad launch failed: %s", cudaGetErrorString(cudaGetLastError()));
   gd.quads = c->d_grid_quads;
   gd.nonfinite = nonfinite;
   if (adjoint) {
-    PSC_CUDA(cudaMemsetAsync(c->d_grad_pairs, 0, np * sizeof(float2), s), "gradient pair reset");
-    gd.grad_pairs = c->d_grad_pairs;
+    int rc = grow(&c->d_grid_grads, &c->grid_grads_cap, nq, "cudaMalloc gradient quads");
+    if (rc) return rc;
+    PSC_CUDA(cudaMemsetAsync(c->d_grid_grads, 0, nq * sizeof(float4), s), "gradient quad reset");
+    gd.grads = c->d_grid_grads;
   }
   return PSC_OK;
 }
@@ -2531,7 +2539,7 @@ int psc_adjoint(psc_ctx* c, const PscDensityGrid* g, const PscView* v, const flo
   if (rc) return rc;
   rc = psc::launch_grid_march(u, vd, gd, true, s);
   if (rc) return fail(rc, "adjoint launch failed: %s", cudaGetErrorString(cudaGetLastError()));
-  rc = psc::launch_grid_fold(gd.grad_pairs, grad_values, gd.nx, gd.ny * gd.nz, s);
+  rc = psc::launch_grid_fold(gd.grads, grad_values, gd.nx, gd.ny, gd.nz, s);
   if (rc) return fail(rc, "gradient fold launch failed: %s", cudaGetErrorString(cudaGetLastError()));
   ++c->launches;
   return PSC_OK;

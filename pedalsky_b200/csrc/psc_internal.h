@@ -158,7 +158,7 @@ struct GridDev {
   const float* values;     // ny x nz x nx, x fastest
   float* grad;             // adjoint: d loss / d values (accumulated)
   uint32_t nx, ny, nz;
-  uint32_t k_cp;           // adjoint checkpoint interval (steps)
+  float fnx, fny, fnz;     // nx, ny, nz, never rounded up
   float min_x, min_z, base;
   float inv_cell_x, inv_cell_y, inv_cell_z;
   float k;                 // density = k * value (density_scale * inv_sigma_bar)
@@ -169,24 +169,27 @@ struct GridDev {
   const float4* target;    // adjoint: target image per pixel of the view
   double* loss;            // adjoint: accumulated loss
   double* grad_scale;      // adjoint: accumulated d loss / d density_scale
-  // the values as (x, z) corner quads: entry (y, zk, xk) holds
-  // v[y][zk-1][xk-1], v[y][zk-1][xk], v[y][zk][xk-1], v[y][zk][xk], zero
-  // outside the grid, zk = 0..nz, xk = 0..nx (launch_grid_quads); the adjoint
-  // adds its gradient into x pairs, entry xk of a (y, z) row for
-  // (x = xk - 1, xk) (grad_pairs), and folds them into grad afterwards
-  // (launch_grid_fold)
+  // the values as (x, z) corner quads: entry (yi, zi, xi) holds v[y][z][x],
+  // v[y][z+1][x], v[y][z][x+1], v[y][z+1][x+1] with y = yi - 2, z = zi - 2,
+  // x = xi - 2, zero outside the grid; yi = 0..ny+3, zi = 0..nz+2,
+  // xi = 0..nx+2 (launch_grid_quads).  The adjoint adds its gradient into an
+  // array of the same form (grads), folded into grad afterwards
+  // (launch_grid_fold).
   const float4* quads;
   const uint32_t* nonfinite;  // 1 when the grid holds an infinity or NaN
-  float2* grad_pairs;
+  float4* grads;
+  uint32_t row;     // entries per row of either array: nx + 3
+  uint32_t origin;  // 0x4B3FFFFE x (plane + row + 1) mod 2^32 (grid_cell)
+  uint64_t plane;   // entries per y plane: (nz + 3) (nx + 3)
 };
 int launch_grid_march(const MarchUniforms& u, const ViewDev& v, const GridDev& g, bool adjoint,
                       cudaStream_t stream);
-// quads[(y (nz + 1) + zk) (nx + 1) + xk] as GridDev::quads from the ny x nz x
-// nx values; *nonfinite = 1 when a value is an infinity or NaN, else 0
-// grad[r nx + x] += gp[r (nx + 1) + x + 1].x + gp[r (nx + 1) + x].y
+// GridDev::quads from the ny x nz x nx values; *nonfinite = 1 when a value is
+// an infinity or NaN, else 0
+// grad += each cell's four entries of grads
 int launch_grid_quads(const float* values, float4* quads, uint32_t* nonfinite, uint32_t nx, uint32_t ny,
                       uint32_t nz, cudaStream_t stream);
-int launch_grid_fold(const float2* grad_pairs, float* grad, uint32_t nx, uint32_t rows, cudaStream_t stream);
+int launch_grid_fold(const float4* grads, float* grad, uint32_t nx, uint32_t ny, uint32_t nz, cudaStream_t stream);
 // d loss / d (base_m, top_m) of layer 0 in the grid form, added to out[0..1]
 // (grid_layer_grad.cu); g.bg / g.target / g.inv_n as for the adjoint.
 int launch_grid_layer_grad(const MarchUniforms& u, const ViewDev& v, const GridDev& g, double* out,
