@@ -21,7 +21,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
-#include "march_fast_body.cuh"
+#include "grid_common.cuh"
 
 namespace psc {
 namespace {
@@ -86,43 +86,36 @@ __device__ __forceinline__ D2 alt_from_d(const MarchUniforms& u, D2 qx, D2 qy, D
   return h0 + num / (r0 + len);
 }
 
-// The grid record's altitude mapping as carried values: base and 1 / cell
-// height (ny / (top - base)).
-struct GridY {
-  D2 base, icy;
-};
+// Whether any of a cell's eight corners holds a value: without one the grid
+// value and its derivatives are 0.
+template <bool WIDE>
+__device__ __forceinline__ bool cell_filled(const GridDev& g, const Cell<WIDE>& c) {
+  const float4 a = __ldg(g.quads + c.i), b = __ldg(g.quads + (c.i + (decltype(c.i))g.plane));
+  const uint32_t bits = __float_as_uint(a.x) | __float_as_uint(a.y) | __float_as_uint(a.z) | __float_as_uint(a.w) |
+                        __float_as_uint(b.x) | __float_as_uint(b.y) | __float_as_uint(b.z) | __float_as_uint(b.w);
+  return (bits << 1) != 0u;  // -0 is empty too
+}
 
-// Trilinear grid value (cell centres, zero outside) at world x / altitude / z.
-__device__ __forceinline__ D2 grid_fetch_d(const GridDev& g, const GridY& gy, D2 x, D2 alt, D2 z) {
-  const D2 fx = (x - g.min_x) * g.inv_cell_x - 0.5f;
-  const D2 fy = (alt - gy.base) * gy.icy - 0.5f;
-  const D2 fz = (z - g.min_z) * g.inv_cell_z - 0.5f;
-  const float cx = floorf(fminf(fmaxf(fx.v, -2.0f), (float)g.nx + 1.0f));
-  const float cy = floorf(fminf(fmaxf(fy.v, -2.0f), (float)g.ny + 1.0f));
-  const float cz = floorf(fminf(fmaxf(fz.v, -2.0f), (float)g.nz + 1.0f));
-  const D2 wx = fx - cx, wy = fy - cy, wz = fz - cz;
-  const int x0 = (int)cx, y0 = (int)cy, z0 = (int)cz;
-  D2 v = dc(0.0f);
-#pragma unroll
-  for (int dy = 0; dy < 2; ++dy) {
-    const int Y = y0 + dy;
-    if (Y < 0 || Y >= (int)g.ny) continue;
-    const D2 fwy = dy ? wy : 1.0f - wy;
-#pragma unroll
-    for (int dz = 0; dz < 2; ++dz) {
-      const int Z = z0 + dz;
-      if (Z < 0 || Z >= (int)g.nz) continue;
-      const D2 wyz = fwy * (dz ? wz : 1.0f - wz);
-      const uint32_t row = ((uint32_t)Y * g.nz + (uint32_t)Z) * g.nx;
-#pragma unroll
-      for (int dx = 0; dx < 2; ++dx) {
-        const int X = x0 + dx;
-        if (X < 0 || X >= (int)g.nx) continue;
-        v = v + (wyz * (dx ? wx : 1.0f - wx)) * __ldg(g.values + row + (uint32_t)X);
-      }
-    }
-  }
-  return v;
+// Grid value and its slopes along the three cell coordinates.
+struct GridSlopes {
+  float v, x, y, z;
+};
+template <bool WIDE>
+__device__ __forceinline__ GridSlopes grid_fetch_slopes(const GridDev& g, const GridPos& p) {
+  const Cell<WIDE> c = grid_cell<WIDE>(g, p);
+  const float4 a = __ldg(g.quads + c.i), b = __ldg(g.quads + (c.i + (decltype(c.i))g.plane));
+  // the quad's lanes are (z, x): 00, 10, 01, 11
+  const float a0 = fmaf(c.wz, a.y - a.x, a.x), a1 = fmaf(c.wz, a.w - a.z, a.z);
+  const float b0 = fmaf(c.wz, b.y - b.x, b.x), b1 = fmaf(c.wz, b.w - b.z, b.z);
+  const float ya = fmaf(c.wx, a1 - a0, a0), yb = fmaf(c.wx, b1 - b0, b0);
+  GridSlopes s;
+  s.v = fmaf(c.wy, yb - ya, ya);
+  s.x = fmaf(c.wy, (b1 - b0) - (a1 - a0), a1 - a0);
+  s.y = yb - ya;
+  const float za = fmaf(c.wx, (a.w - a.z) - (a.y - a.x), a.y - a.x);
+  const float zb = fmaf(c.wx, (b.w - b.z) - (b.y - b.x), b.y - b.x);
+  s.z = fmaf(c.wy, zb - za, za);
+  return s;
 }
 
 // Bilinear clamp-to-edge lookup of the RGB channels of a float4 LUT at
@@ -209,6 +202,16 @@ __device__ __forceinline__ D2 shell_distance(const MarchUniforms& u, const Layer
 
 // One ray of the grid march (grid_pixel in grid_march.cu) carried with its
 // derivatives; returns this pixel's d loss / d base and d loss / d top.
+//
+// A grid value's derivatives are its slopes along the three cell coordinates
+// times theirs, so the eight weights are not carried.  Samples whose eight
+// corners are empty add nothing and are passed over.  The sums cancel (a
+// sample near the vertical through the world's origin turns its azimuth fast,
+// and slopes jump at cell borders), so positions keep the operations of the
+// carried form.  Bound by instructions (164 registers, 3 CTAs per SM): 512^2
+// rays, 96 + 6 steps, 256x64x256 cells at 13 % fill 2951 -> 356 us; bounded
+// to 128 or 96 registers it spills and takes 362 or 412 us.
+template <bool WIDE>
 __device__ __forceinline__ void layer_grad_pixel(const MarchUniforms& u, const ViewDev& v, const GridDev& g,
                                                  uint32_t px, uint32_t py, float& d_base, float& d_top) {
   d_base = d_top = 0.0f;
@@ -249,7 +252,9 @@ __device__ __forceinline__ void layer_grad_pixel(const MarchUniforms& u, const V
   const D2 base = {L.base_m, 1.0f, 0.0f}, top = {L.top_m, 0.0f, 1.0f};
   const D2 thick = top - base;
   const D2 inv_thick = dc(1.0f) / dmax(thick, 1.0f);
-  const GridY gy{base, dc((float)g.ny) / dmax(thick, 1.0f)};
+  // cells per metre of altitude, ny / (top - base)
+  const D2 icy = dc((float)g.ny) / dmax(thick, 1.0f);
+  const bool every = __ldg(g.nonfinite) != 0u;  // as in grid_pixel
 
   D2 Lc[3] = {dc(0.0f), dc(0.0f), dc(0.0f)}, T[3] = {dc(1.0f), dc(1.0f), dc(1.0f)};
   if (hit) {
@@ -258,64 +263,95 @@ __device__ __forceinline__ void layer_grad_pixel(const MarchUniforms& u, const V
     const D2 t1 = shell_distance(u, L, oc, rs.dird, rs.t1[0]);
     const D2 step = (t1 - t0) * (1.0f / (float)u.cloud_steps);
     const D2 r0 = dc(rs.r0), cvv = dc(rs.cos_view), h0 = dc(rs.h0);
-    for (uint32_t s = 0; s < u.cloud_steps; ++s) {
-      const D2 t = t0 + step * ((float)s + jitter);
-      const D2 p3x = t * dx + cx, p3y = t * dy + cy, p3z = t * dz + cz;
-      const D2 alt = alt_from_d(u, p3x, p3y, p3z, r0, cvv, h0, t);
-      const D2 inv_r = dc(1.0f) / (alt + u.planet_r);
-      const D2 ux = p3x * inv_r, uy = (p3y + u.planet_r) * inv_r, uz = p3z * inv_r;
-      const D2 gv = grid_fetch_d(g, gy, p3x, alt, p3z);
-      // light march toward the sun (light_geo / light_sum)
-      const D2 lr0 = alt + u.planet_r;
-      const D2 lcv = ux * u.sun[0] + uy * u.sun[1] + uz * u.sun[2];
-      const D2 delta = dmax((top - alt) * u.inv_cos_sun, 1.0f) * (1.0f / (float)u.light_steps);
-      D2 gl = dc(0.0f);
-      for (uint32_t j = 0; j < u.light_steps; ++j) {
-        const D2 tj = delta * ((float)j + 0.5f);
-        const D2 qx = p3x + tj * u.sun[0], qy = p3y + tj * u.sun[1], qz = p3z + tj * u.sun[2];
-        gl = gl + grid_fetch_d(g, gy, qx, alt_from_d(u, qx, qy, qz, lr0, lcv, alt, tj), qz);
-      }
-      gl = gl * delta;
-      const D2 rho = gv * g.k, od = gl * g.k;
-      // lighting: sun factor, ambient (+ lightning)
-      D2 ts[3], sky[3];
-      lut_lookups_d(u, alt, ux, uy, uz, ts, sky);
-      const D2 h = dclamp((alt - base) * inv_thick, 0.0f, 1.0f);
-      const D2 ag = (h * 0.7f + 0.3f) * u.ambient;
-      float lgt[3] = {0.0f, 0.0f, 0.0f};
-      D2 lw = dc(0.0f);
-      if (u.lightning_radius > 0.0f) {
-        const D2 ddx = p3x - u.lightning_origin_x, ddz = p3z - u.lightning_origin_z;
-        const D2 fo = dclamp(1.0f - dsqrt(ddx * ddx + ddz * ddz) * (1.0f / u.lightning_radius), 0.0f, 1.0f);
-        lw = fo * fo * (3.0f - 2.0f * fo);
-        lgt[0] = u.lightning_rgb[0];
-        lgt[1] = u.lightning_rgb[1];
-        lgt[2] = u.lightning_rgb[2];
-      }
+    constexpr uint32_t kAhead = 4;  // steps whose cells are looked at together, as in grid_pixel
+    bool done = false;
+    for (uint32_t s0 = 0; s0 < u.cloud_steps && !done; s0 += kAhead) {
+      uint32_t todo = 0;
 #pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        // source X(od) = sun * Beer-powder * octaves + ambient (grid_march.cu:source)
-        D2 S = dc(0.0f), B = dc(1.0f);
-#pragma unroll
-        for (int n = 0; n < kMaxOct; ++n) {
-          if (n < (int)u.octaves) {
-            const D2 e = dexp(od * (-st[c] * u.bpow[n]));
-            if (n == 0) B = e;
-            S = S + e * coef[n];
-          }
+      for (uint32_t k = 0; k < kAhead; ++k) {
+        // the values of the carried position below, in the same operations:
+        // a sample must be looked at in the cell it is evaluated in
+        const float t = t0.v + step.v * ((float)(s0 + k) + jitter);
+        const float x = t * dx + cx, y = t * dy + cy, z = t * dz + cz, yy = y + u.planet_r;
+        const float num = t * (2.0f * rs.r0 * rs.cos_view + t), len = sqrtf(fmaxf(x * x + yy * yy + z * z, 0.0f));
+        const float alt = rs.h0 + num * (1.0f / (rs.r0 + len));
+        const GridPos q{(x - g.min_x) * g.inv_cell_x - 0.5f, (alt - base.v) * icy.v - 0.5f, (z - g.min_z) * g.inv_cell_z - 0.5f};
+        const bool filled = cell_filled<WIDE>(g, grid_cell<WIDE>(g, q));
+        todo |= (s0 + k < u.cloud_steps && (filled || every)) ? 1u << k : 0u;
+      }
+      while (todo) {
+        const uint32_t s = s0 + (uint32_t)__ffs((int)todo) - 1u;
+        todo &= todo - 1u;
+        const D2 t = t0 + step * ((float)s + jitter);
+        const D2 p3x = t * dx + cx, p3y = t * dy + cy, p3z = t * dz + cz;
+        const D2 alt = alt_from_d(u, p3x, p3y, p3z, r0, cvv, h0, t);
+        const D2 inv_r = dc(1.0f) / (alt + u.planet_r);
+        const D2 ux = p3x * inv_r, uy = (p3y + u.planet_r) * inv_r, uz = p3z * inv_r;
+        // grid value at a point whose altitude is `h`
+        auto value = [&](D2 x, D2 h, D2 z) {
+          const D2 y = (h - base) * icy - 0.5f;
+          const GridSlopes f =
+              grid_fetch_slopes<WIDE>(g, GridPos{(x.v - g.min_x) * g.inv_cell_x - 0.5f, y.v, (z.v - g.min_z) * g.inv_cell_z - 0.5f});
+          const float kx = f.x * g.inv_cell_x, kz = f.z * g.inv_cell_z;
+          return D2{f.v, fmaf(kx, x.a, fmaf(f.y, y.a, kz * z.a)), fmaf(kx, x.b, fmaf(f.y, y.b, kz * z.b))};
+        };
+        const D2 gv = value(p3x, alt, p3z);
+        // light march toward the sun (light_geo / light_sum)
+        const D2 lr0 = alt + u.planet_r;
+        const D2 lcv = ux * u.sun[0] + uy * u.sun[1] + uz * u.sun[2];
+        const D2 delta = dmax((top - alt) * u.inv_cos_sun, 1.0f) * (1.0f / (float)u.light_steps);
+        D2 gl = dc(0.0f);
+#pragma unroll 1
+        for (uint32_t j = 0; j < u.light_steps; ++j) {
+          const D2 tj = delta * ((float)j + 0.5f);
+          const D2 qx = p3x + tj * u.sun[0], qy = p3y + tj * u.sun[1], qz = p3z + tj * u.sun[2];
+          gl = gl + value(qx, alt_from_d(u, qx, qy, qz, lr0, lcv, alt, tj), qz);
         }
-        S = S * (ts[c] * u.sun_illum[c]);
-        const D2 P = 1.0f - B * B;
-        const D2 E = B + (B * P * 2.0f - B) * u.powder;
-        const D2 X = S * E + sky[c] * ag + lw * lgt[c];
-        const D2 x = rho * step * st[c];
-        const float e = __expf(-x.v);
-        const D2 om = one_minus_exp_neg_d(x, e);  // 1 - exp(-x)
-        // the step integral rho ss X step (1 - e^-x) / x = ss X (1 - e^-x) / st
-        Lc[c] = Lc[c] + T[c] * X * om * (ss[c] / st[c]);
-        T[c] = T[c] * D2{e, -x.a * e, -x.b * e};
+        gl = gl * delta;
+        const D2 rho = gv * g.k, od = gl * g.k;
+        // lighting: sun factor, ambient (+ lightning)
+        D2 ts[3], sky[3];
+        lut_lookups_d(u, alt, ux, uy, uz, ts, sky);
+        const D2 h = dclamp((alt - base) * inv_thick, 0.0f, 1.0f);
+        const D2 ag = (h * 0.7f + 0.3f) * u.ambient;
+        float lgt[3] = {0.0f, 0.0f, 0.0f};
+        D2 lw = dc(0.0f);
+        if (u.lightning_radius > 0.0f) {
+          const D2 ddx = p3x - u.lightning_origin_x, ddz = p3z - u.lightning_origin_z;
+          const D2 fo = dclamp(1.0f - dsqrt(ddx * ddx + ddz * ddz) * (1.0f / u.lightning_radius), 0.0f, 1.0f);
+          lw = fo * fo * (3.0f - 2.0f * fo);
+          lgt[0] = u.lightning_rgb[0];
+          lgt[1] = u.lightning_rgb[1];
+          lgt[2] = u.lightning_rgb[2];
+        }
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          // source X(od) = sun * Beer-powder * octaves + ambient (grid_march.cu:source)
+          D2 S = dc(0.0f), B = dc(1.0f);
+#pragma unroll
+          for (int n = 0; n < kMaxOct; ++n) {
+            if (n < (int)u.octaves) {
+              const D2 e = dexp(od * (-st[c] * u.bpow[n]));
+              if (n == 0) B = e;
+              S = S + e * coef[n];
+            }
+          }
+          S = S * (ts[c] * u.sun_illum[c]);
+          const D2 P = 1.0f - B * B;
+          const D2 E = B + (B * P * 2.0f - B) * u.powder;
+          const D2 X = S * E + sky[c] * ag + lw * lgt[c];
+          const D2 x = rho * step * st[c];
+          const float e = __expf(-x.v);
+          const D2 om = one_minus_exp_neg_d(x, e);  // 1 - exp(-x)
+          // the step integral rho ss X step (1 - e^-x) / x = ss X (1 - e^-x) / st
+          Lc[c] = Lc[c] + T[c] * X * om * (ss[c] / st[c]);
+          T[c] = T[c] * D2{e, -x.a * e, -x.b * e};
+        }
+        if (fmaxf(T[0].v, fmaxf(T[1].v, T[2].v)) < g.exit_t) {
+          done = true;
+          break;
+        }
       }
-      if (fmaxf(T[0].v, fmaxf(T[1].v, T[2].v)) < g.exit_t) break;
     }
   }
   const size_t idx = (size_t)py * v.width + px;
@@ -336,6 +372,7 @@ __device__ __forceinline__ double warp_sum(double x) {
   return x;
 }
 
+template <bool WIDE>
 __global__ void __launch_bounds__(kThreads) k_grid_layer_grad(const __grid_constant__ MarchUniforms u,
                                                               const __grid_constant__ ViewDev v,
                                                               const __grid_constant__ GridDev g,
@@ -344,7 +381,7 @@ __global__ void __launch_bounds__(kThreads) k_grid_layer_grad(const __grid_const
   const uint32_t px = blockIdx.x * kTileW + (warp & 1u) * 8u + (lane & 7u);
   const uint32_t py = blockIdx.y * kTileH + (warp >> 1) * 4u + (lane >> 3);
   float db = 0.0f, dt = 0.0f;
-  if (px < v.width && py < v.height) layer_grad_pixel(u, v, g, px, py, db, dt);
+  if (px < v.width && py < v.height) layer_grad_pixel<WIDE>(u, v, g, px, py, db, dt);
   __shared__ double s_red[2][kThreads / 32];
   const double sb = warp_sum((double)db), st = warp_sum((double)dt);
   if (lane == 0) {
@@ -368,9 +405,13 @@ __global__ void __launch_bounds__(kThreads) k_grid_layer_grad(const __grid_const
 
 int launch_grid_layer_grad(const MarchUniforms& u, const ViewDev& v, const GridDev& g, double* out,
                            cudaStream_t s) {
+  if (!g.quads) return PSC_ERR_INVALID_ARGUMENT;
   if (u.octaves == 0 || u.octaves > (uint32_t)kMaxOct) return PSC_ERR_UNSUPPORTED;
   const dim3 grid((v.width + kTileW - 1) / kTileW, (v.height + kTileH - 1) / kTileH);
-  k_grid_layer_grad<<<grid, kThreads, 0, s>>>(u, v, g, out);
+  if (grid_wide(g))
+    k_grid_layer_grad<true><<<grid, kThreads, 0, s>>>(u, v, g, out);
+  else
+    k_grid_layer_grad<false><<<grid, kThreads, 0, s>>>(u, v, g, out);
   return cudaGetLastError() == cudaSuccess ? PSC_OK : PSC_ERR_CUDA;
 }
 

@@ -2565,6 +2565,8 @@ int psc_layer_gradient(psc_ctx* c, const PscDensityGrid* g, const PscView* v, co
   u.tex_sky = 0;
   gd.bg = reinterpret_cast<const float4*>(background);
   gd.target = reinterpret_cast<const float4*>(target);
+  rc = stage_grid_layout(c, gd, false, static_cast<cudaStream_t>(stream));
+  if (rc) return rc;
   rc = psc::launch_grid_layer_grad(u, vd, gd, grad_base_top, static_cast<cudaStream_t>(stream));
   if (rc) return fail(rc, "layer-gradient launch failed: %s", cudaGetErrorString(cudaGetLastError()));
   ++c->launches;

@@ -123,3 +123,30 @@ def test_wide_grid_matches_narrow_grid(oracle, oracle_noise):
     assert np.linalg.norm(a - b) <= 1e-4 * np.linalg.norm(a)
     assert abs(ga - gb) <= 1e-4 * abs(ga)
     np.testing.assert_allclose(ab, aa, rtol=1e-4)
+
+
+@pytest.mark.parametrize("shape,steps,light", [((5, 3, 7), 23, 6), ((33, 9, 2), 40, 5), ((64, 1, 65), 17, 1)])
+def test_range_gradient_of_an_embedded_grid(oracle, oracle_noise, shape, steps, light):
+    """A ring of empty cells around a grid (its extent grown by as much) is
+    the same cloud, so the gradient in the layer's base and top is the same.
+    The grid's slopes jump at cell borders and the two sets of cell
+    coordinates round apart by about 1e-5 cells: of the 3e5 taps of this view
+    a few change cells, each worth at most 1e-3 of the sum: 1e-2."""
+    torch, sc, luts, G, spec, sub, P, tgt = _problem(oracle, oracle_noise, shape, steps, light, 35.0, 0.5)
+    ring = np.pad(G, ((0, 0), (1, 1), (1, 1)))
+    cx, cz = spec["size_x_m"] / shape[0], spec["size_z_m"] / shape[2]
+    grown = dict(spec, min_x_m=spec["min_x_m"] - cx, min_z_m=spec["min_z_m"] - cz, size_x_m=spec["size_x_m"] + 2 * cx,
+                 size_z_m=spec["size_z_m"] + 2 * cz)
+    got = []
+    try:
+        for Q in (P, GR.GridProblem(sc, ring, spec=grown)):
+            Q.set_target(tgt)
+            out = torch.zeros(2, dtype=torch.float64, device="cuda:0")
+            Q.layer_gradient(sub.handle, out)
+            torch.cuda.synchronize()
+            got.append(out.cpu().numpy())
+    finally:
+        sub.close()
+    print(shape, got)
+    assert np.abs(got[0]).min() > 0
+    assert np.linalg.norm(got[0] - got[1]) <= 1e-2 * np.linalg.norm(got[0])
