@@ -106,20 +106,6 @@ __device__ __forceinline__ float4 trilinear_texel(const void* vol, float x, floa
   return r;
 }
 
-// floor(x) and its integer bits for |x| < 2^22: one round-down add puts
-// 1.5 * 2^23 + floor(x) in a float whose low mantissa bits are floor(x)
-// (two's complement, so masks wrap negative indices), and subtracting the
-// constant back is exact.  Larger |x| (millions of texels, far beyond any
-// ray here) still yields masked, in-bounds indices.
-struct FloorBits {
-  float f;
-  uint32_t i;
-};
-__device__ __forceinline__ FloorBits floor_bits(float x) {
-  const float s = __fadd_rd(x, 12582912.0f);
-  return {s - 12582912.0f, __float_as_uint(s)};
-}
-
 __device__ __forceinline__ float2 h2f(uint32_t w) {
   return __half22float2(*reinterpret_cast<const __half2*>(&w));
 }
@@ -219,8 +205,11 @@ __device__ __forceinline__ float2 base_tap(const MarchUniforms& u, float ax, flo
                         az * u.inv_base_scale);
     } else {
       const float k = u.base_texel_scale;
-      b = trilinear_texel<ST, 128>(u.noise_base, fmaf(ax, k, -0.5f), fmaf(ay, k, -0.5f),
-                                   fmaf(az, k, -0.5f), u.noise_scale);
+      if constexpr (ST == PSC_STORAGE_U8)
+        b = trilinear_quad_u8<128>(u.base_quad, fmaf(ax, k, -0.5f), fmaf(ay, k, -0.5f), fmaf(az, k, -0.5f));
+      else
+        b = trilinear_texel<ST, 128>(u.noise_base, fmaf(ax, k, -0.5f), fmaf(ay, k, -0.5f),
+                                     fmaf(az, k, -0.5f), u.noise_scale);
     }
     return make_float2(b.x, fmaf(b.w, 0.125f, fmaf(b.z, 0.25f, b.y * 0.625f)));
   }
@@ -244,8 +233,11 @@ __device__ __forceinline__ float detail_tap(const MarchUniforms& u, float dx, fl
                         dz * u.inv_detail_scale);
     } else {
       const float k = u.detail_texel_scale;
-      d = trilinear_texel<ST, 32>(u.noise_detail, fmaf(dx, k, -0.5f), fmaf(dy, k, -0.5f),
-                                  fmaf(dz, k, -0.5f), u.noise_scale);
+      if constexpr (ST == PSC_STORAGE_U8)
+        d = trilinear_quad_u8<32>(u.detail_quad8, fmaf(dx, k, -0.5f), fmaf(dy, k, -0.5f), fmaf(dz, k, -0.5f));
+      else
+        d = trilinear_texel<ST, 32>(u.noise_detail, fmaf(dx, k, -0.5f), fmaf(dy, k, -0.5f),
+                                    fmaf(dz, k, -0.5f), u.noise_scale);
     }
     return fmaf(d.z, 0.125f, fmaf(d.y, 0.25f, d.x * 0.625f));
   }
@@ -681,49 +673,6 @@ __device__ __forceinline__ float weather_fast(const MarchUniforms& u, float uu, 
   const float a = lerpf(__ldg(u.weather + y0 * W + x0), __ldg(u.weather + y0 * W + x1), wx);
   const float b = lerpf(__ldg(u.weather + y1 * W + x0), __ldg(u.weather + y1 * W + x1), wx);
   return lerpf(a, b, wy);
-}
-
-// The primary steps of a ray's layer segment that can pass the profile test
-// (no type grid): those whose altitude lies in the layer's band
-// [live_lo, live_hi] (LayerConst), found from the ray's geometry instead of
-// stepping through the rest.  Along the ray, |o + t d| = R + a at
-// t = tv -/+ sqrt((R + a)^2 - rp^2) with tv = -r0 cos(up, d) and rp the
-// line's closest distance to the planet centre, so the altitude stays at or
-// below a_hi on [tv - sqrt(q_hi), tv + sqrt(q_hi)] and falls below a_lo only
-// inside (tv - sqrt(q_lo), tv + sqrt(q_lo)); the hull of what remains in
-// [t0, t1] becomes step indices.  In FP64 from the FP32 r0 and cos(up, d)
-// the ray carries (their rounding moves t by about 1 m at most), with the
-// band widened by 3 m more and the index range by 2-3 steps: every step that
-// could pass the test is inside [s_begin, s_end), and the steps outside add
-// nothing and leave the transmittance as it is, so skipping them is exact.
-// Returns false when no step of the segment can pass.
-__device__ __forceinline__ bool live_step_range(float r0f, float ray_B, const LayerConst& L, float R,
-                                                float t0, float t1, float step, float jitter,
-                                                uint32_t n, uint32_t& s_begin, uint32_t& s_end) {
-  const double r0 = r0f, cv = (double)ray_B / (2.0 * fmax(r0, 1.0));
-  const double tv = -r0 * cv;
-  const double rp2 = r0 * r0 * fmax(1.0 - cv * cv, 0.0);
-  const double rh = (double)R + ((double)L.live_hi + 3.0), rl = (double)R + ((double)L.live_lo - 3.0);
-  const double qh = rh * rh - rp2;
-  if (qh < 0.0) return false;  // the line stays above the band
-  const double sh = sqrt(qh);
-  double lo = fmax((double)t0, tv - sh), hi = fmin((double)t1, tv + sh);
-  if (lo > hi) return false;
-  const double ql = rl * rl - rp2;
-  if (ql > 0.0) {  // the open interval where the altitude is below the band
-    const double sl = sqrt(ql), c = tv - sl, d = tv + sl;
-    const bool p1 = lo <= fmin(hi, c), p2 = fmax(lo, d) <= hi;
-    if (!p1 && !p2) return false;
-    const double nlo = p1 ? lo : fmax(lo, d), nhi = p2 ? hi : fmin(hi, c);
-    lo = nlo;
-    hi = nhi;
-  }
-  const double is = 1.0 / (double)step;
-  const double fb = floor((lo - (double)t0) * is - (double)jitter) - 2.0;
-  const double fe = ceil((hi - (double)t0) * is - (double)jitter) + 3.0;
-  s_begin = fb <= 0.0 ? 0u : (fb >= (double)n ? n : (uint32_t)fb);
-  s_end = fe <= 0.0 ? 0u : (fe >= (double)n ? n : (uint32_t)fe);
-  return s_begin < s_end;
 }
 
 // 1 - exp(-y) without cancellation for small y.

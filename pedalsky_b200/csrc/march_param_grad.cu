@@ -357,8 +357,11 @@ struct LayerD {
 template <int ST, bool LIGHT>
 __device__ DV density_d(const MarchUniforms& u, const LayerConst& L, const LayerD* cd, const DV3& p, const DV& alt,
                         const DV& wr, uint32_t type) {
-  if (!cd)
-    return dc(density_at<ST, PSC_FILTER_EXACT, LIGHT>(u, L, p.x.v, p.y.v, p.z.v, alt.v, wr.v, type, nullptr));
+  if (!cd) {
+    const Cover cov = cover_of(L, wr.v);
+    return dc(LIGHT ? density_light_at<ST, PSC_FILTER_EXACT>(u, L, p.x.v, p.y.v, p.z.v, alt.v, cov, type, nullptr)
+                    : density_primary_at<ST, PSC_FILTER_EXACT>(u, L, p.x.v, p.y.v, p.z.v, alt.v, cov, type, nullptr));
+  }
   const LayerD& D = *cd;
   const DV h = (alt - D.base) / dmax(D.top - D.base, 1.0f);
   if (h.v < 0.0f || h.v > 1.0f) return dc(0.0f);

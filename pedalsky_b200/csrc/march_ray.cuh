@@ -2,7 +2,8 @@
 // (compute_view_ray, shaders/common/math.wgsl:23-33), the depth clip
 // (cloud_march.wgsl:764-775), the per-layer shell intersection
 // (ray_layer_intersect, cloud_march.wgsl:370-416) and the stable sort of the
-// hit layers by entry distance (:796-806).  All in FP64: at planet radius
+// hit layers by entry distance (:796-806), and the range of a layer's steps
+// that can hold cloud.  All in FP64: at planet radius
 // (6.36e6 m) the FP32 form |oc|^2 - r^2 cancels catastrophically and moves
 // the layer entry by metres, which the detail noise (25 m texels) resolves.
 #pragma once
@@ -131,6 +132,49 @@ __device__ void setup_ray(const MarchUniforms& u, const ViewDev& v, uint32_t px,
       rs.order |= (uint32_t)i << (4 * rank);
     }
   }
+}
+
+// The primary steps of a ray's layer segment that can pass the profile test
+// (no type grid): those whose altitude lies in the layer's band
+// [live_lo, live_hi] (LayerConst), found from the ray's geometry instead of
+// stepping through the rest.  Along the ray, |o + t d| = R + a at
+// t = tv -/+ sqrt((R + a)^2 - rp^2) with tv = -r0 cos(up, d) and rp the
+// line's closest distance to the planet centre, so the altitude stays at or
+// below a_hi on [tv - sqrt(q_hi), tv + sqrt(q_hi)] and falls below a_lo only
+// inside (tv - sqrt(q_lo), tv + sqrt(q_lo)); the hull of what remains in
+// [t0, t1] becomes step indices.  In FP64 from the FP32 r0 and cos(up, d)
+// the ray carries (their rounding moves t by about 1 m at most), with the
+// band widened by 3 m more and the index range by 2-3 steps: every step that
+// could pass the test is inside [s_begin, s_end), and the steps outside add
+// nothing and leave the transmittance as it is, so skipping them is exact.
+// Returns false when no step of the segment can pass.
+__device__ __forceinline__ bool live_step_range(float r0f, float ray_B, const LayerConst& L, float R,
+                                                float t0, float t1, float step, float jitter,
+                                                uint32_t n, uint32_t& s_begin, uint32_t& s_end) {
+  const double r0 = r0f, cv = (double)ray_B / (2.0 * fmax(r0, 1.0));
+  const double tv = -r0 * cv;
+  const double rp2 = r0 * r0 * fmax(1.0 - cv * cv, 0.0);
+  const double rh = (double)R + ((double)L.live_hi + 3.0), rl = (double)R + ((double)L.live_lo - 3.0);
+  const double qh = rh * rh - rp2;
+  if (qh < 0.0) return false;  // the line stays above the band
+  const double sh = sqrt(qh);
+  double lo = fmax((double)t0, tv - sh), hi = fmin((double)t1, tv + sh);
+  if (lo > hi) return false;
+  const double ql = rl * rl - rp2;
+  if (ql > 0.0) {  // the open interval where the altitude is below the band
+    const double sl = sqrt(ql), c = tv - sl, d = tv + sl;
+    const bool p1 = lo <= fmin(hi, c), p2 = fmax(lo, d) <= hi;
+    if (!p1 && !p2) return false;
+    const double nlo = p1 ? lo : fmax(lo, d), nhi = p2 ? hi : fmin(hi, c);
+    lo = nlo;
+    hi = nhi;
+  }
+  const double is = 1.0 / (double)step;
+  const double fb = floor((lo - (double)t0) * is - (double)jitter) - 2.0;
+  const double fe = ceil((hi - (double)t0) * is - (double)jitter) + 3.0;
+  s_begin = fb <= 0.0 ? 0u : (fb >= (double)n ? n : (uint32_t)fb);
+  s_end = fe <= 0.0 ? 0u : (fe >= (double)n ? n : (uint32_t)fe);
+  return s_begin < s_end;
 }
 
 }  // namespace

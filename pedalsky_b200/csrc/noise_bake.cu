@@ -272,6 +272,19 @@ __global__ void k_fold_detail(const uint32_t* __restrict__ src, uint16_t* __rest
                        fold_detail_texel(src[row1 + x]) | (fold_detail_texel(src[row1 + x1]) << 16));
 }
 
+// RGBA8 volume (n^3, n a power of two) as the 2x2 (x, y) footprint of slab z
+// per entry, repeat-wrapped: a trilinear tap is two 16-byte loads instead of
+// eight 4-byte ones (the exact FAST march of an 853x479 view, two layers, 192
+// steps: 3.12 -> 2.41 ms).
+__global__ void k_quads_u8(const uint32_t* __restrict__ src, uint4* __restrict__ quad, uint32_t n) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n * n * n) return;
+  const uint32_t x = i & (n - 1u), y = (i / n) & (n - 1u), slab = i - (y * n + x);
+  const uint32_t x1 = (x + 1u) & (n - 1u), y1 = (y + 1u) & (n - 1u);
+  const uint32_t* const s = src + slab;
+  quad[i] = make_uint4(s[y * n + x], s[y * n + x1], s[y1 * n + x], s[y1 * n + x1]);
+}
+
 // Curl tile (128^2 RG8) as 2x2 quads of (R, G) half pairs, repeat-wrapped:
 // a bilinear curl tap is one 16-byte load.  Bytes are exact in FP16.
 __global__ void k_curl_quads(const uint16_t* __restrict__ src, uint4* __restrict__ quad) {
@@ -290,6 +303,11 @@ __global__ void k_curl_quads(const uint16_t* __restrict__ src, uint4* __restrict
 
 int launch_curl_quads(const uint8_t* curl, uint4* quad, cudaStream_t s) {
   k_curl_quads<<<128u * 128u / 256u, 256, 0, s>>>(reinterpret_cast<const uint16_t*>(curl), quad);
+  return cudaGetLastError() == cudaSuccess ? PSC_OK : PSC_ERR_CUDA;
+}
+
+int launch_quads_u8(const uint8_t* src, uint4* quad, uint32_t n, cudaStream_t s) {
+  k_quads_u8<<<(n * n * n + 255u) / 256u, 256, 0, s>>>(reinterpret_cast<const uint32_t*>(src), quad, n);
   return cudaGetLastError() == cudaSuccess ? PSC_OK : PSC_ERR_CUDA;
 }
 

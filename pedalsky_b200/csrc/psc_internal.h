@@ -133,10 +133,12 @@ struct alignas(16) MarchUniforms {
   const float4* lut_sky;       // 192x108
   const float4* lut_ap;        // 32x32x64
   cudaTextureObject_t tex_base, tex_detail;  // PSC_FILTER_TEXTURE only
-  // F16 storage in the FAST schedule: channel-folded volumes (R, fbm) and
-  // (detail fbm) as 2x2 quads per entry (noise_bake.cu:k_fold_*)
+  // the noise volumes as 2x2 (x, y) quads per entry: F16 storage (FAST
+  // schedule) the channel-folded (R, fbm) and (detail fbm)
+  // (noise_bake.cu:k_fold_*), U8 storage the RGBA8 texels (k_quads_u8)
   const uint4* base_quad;
-  const uint2* detail_quad;
+  const uint2* detail_quad;    // F16
+  const uint4* detail_quad8;   // U8
   const uint4* curl_quad;      // FAST schedule: curl tile as 2x2 (R, G) half quads
   // transmittance / sky-view LUTs through the texture unit; 0 = plain loads
   cudaTextureObject_t tex_trans, tex_sky;
@@ -256,6 +258,8 @@ int launch_march_fast_tally(const MarchUniforms& u, const ViewDev& v, const PscM
                             unsigned long long* counts, cudaStream_t stream);
 int launch_composite(const float4* l, const float4* t, float4* hdr, uint32_t n,
                      cudaStream_t stream);
+// RGBA8 volumes of n^3 texels (n a power of two) as 2x2 quads per entry.
+int launch_quads_u8(const uint8_t* src, uint4* quad, uint32_t n, cudaStream_t stream);
 // Noise bakes (noise_bake.cu), synchronous on `stream`.
 int launch_noise_bakes(uint8_t* base, uint8_t* detail, uint8_t* curl, cudaStream_t stream);
 // True when a march over these n uniform blocks needs the FAST kernels' full
