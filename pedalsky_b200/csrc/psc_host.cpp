@@ -1402,45 +1402,41 @@ int psc_generate_blue_noise(uint8_t* out) {
   for (int dy = -rad; dy <= rad; ++dy)
     for (int dx = -rad; dx <= rad; ++dx)
       kern[(dy + rad) * 13 + (dx + rad)] = std::exp(-(float)(dx * dx + dy * dy) * k) * 1.0f;
-  std::vector<float> energy(N, 0.0f);
+  std::vector<float> energy(N, 0.0f);  // of the free cells; a placed one is out of the search at infinity
   std::vector<uint32_t> rank(N, 0);
-  std::vector<uint8_t> placed(N, 0);
   // Each step places the free cell of least energy, the first in row-major
   // order.  Energies only grow, so a row's least cell changes only when that
   // cell itself is splatted or placed: kept per row, a step looks at 64 row
   // minima and rescans the few rows whose own was touched, instead of all
-  // 4096 cells (25 to 50 ms for the tile, by code alignment; now 2 ms).
-  std::vector<int> row_best(S, 0);
+  // 4096 cells (25 to 50 ms for the tile, by code alignment; now 4 ms).
+  std::vector<int> row_at(S, 0);
+  std::vector<float> row_min(S, 0.0f);
   auto rescan = [&](int y) {
-    int at = -1;
-    float be = INFINITY;
-    for (int x = 0; x < S; ++x)
-      if (!placed[y * S + x] && energy[y * S + x] < be) {
-        be = energy[y * S + x];
-        at = x;
-      }
-    row_best[y] = at;
+    const float* const e = &energy[(size_t)y * S];
+    float m[8];
+    for (int j = 0; j < 8; ++j) m[j] = e[j];
+    for (int x = 8; x < S; x += 8)
+      for (int j = 0; j < 8; ++j) m[j] = e[x + j] < m[j] ? e[x + j] : m[j];
+    float least = m[0];
+    for (int j = 1; j < 8; ++j) least = m[j] < least ? m[j] : least;
+    int x = 0;
+    while (e[x] != least) ++x;
+    row_at[y] = x;
+    row_min[y] = least;
   };
   for (int step = 0; step < N; ++step) {
-    int best = 0;
-    float be = INFINITY;
-    for (int y = 0; y < S; ++y)
-      if (row_best[y] >= 0 && energy[y * S + row_best[y]] < be) {
-        best = y * S + row_best[y];
-        be = energy[best];
-      }
-    placed[best] = 1;
-    rank[best] = (uint32_t)step;
-    const int cx = best % S, cy = best / S;
+    int cy = 0;
+    for (int y = 1; y < S; ++y)
+      if (row_min[y] < row_min[cy]) cy = y;
+    const int cx = row_at[cy];
+    rank[cy * S + cx] = (uint32_t)step;
+    energy[cy * S + cx] = INFINITY;
     for (int dy = -rad; dy <= rad; ++dy) {
-      const int yy = ((cy + dy) % S + S) % S;
-      bool touched = false;
-      for (int dx = -rad; dx <= rad; ++dx) {
-        const int xx = ((cx + dx) % S + S) % S;
-        energy[yy * S + xx] += kern[(dy + rad) * 13 + (dx + rad)];
-        touched = touched || xx == row_best[yy];
-      }
-      if (touched) rescan(yy);
+      const int yy = (cy + dy) & (S - 1);
+      float* const e = &energy[(size_t)yy * S];
+      const float* const k = kern + (dy + rad) * 13;
+      for (int i = 0; i < 13; ++i) e[(cx + i - rad) & (S - 1)] += k[i];
+      if (((row_at[yy] - cx + rad) & (S - 1)) < 13) rescan(yy);  // its least cell was splatted
     }
   }
   const float maxr = (float)(N - 1);
@@ -1675,11 +1671,16 @@ int psc_bake_noise(psc_ctx* c) {
   if (!c->d_base_u8) PSC_CUDA(cudaMalloc(&c->d_base_u8, 128u * 128u * 128u * 4u), "cudaMalloc base");
   if (!c->d_detail_u8) PSC_CUDA(cudaMalloc(&c->d_detail_u8, 32u * 32u * 32u * 4u), "cudaMalloc detail");
   if (!c->d_curl) PSC_CUDA(cudaMalloc(&c->d_curl, 128u * 128u * 2u), "cudaMalloc curl");
-  if (psc::launch_noise_bakes(c->d_base_u8, c->d_detail_u8, c->d_curl, 0))
-    return fail(PSC_ERR_CUDA, "noise bake failed: %s", cudaGetErrorString(cudaGetLastError()));
-  c->have_base = c->have_detail = c->have_curl = true;
+  float4* cells = nullptr;
+  PSC_CUDA(cudaMalloc(&cells, psc::noise_cells_bytes()), "cudaMalloc noise cells");
+  const int baked = psc::launch_noise_bakes(cells, c->d_base_u8, c->d_detail_u8, c->d_curl, 0);
   std::vector<uint8_t> blue(64 * 64);
-  psc_generate_blue_noise(blue.data());
+  psc_generate_blue_noise(blue.data());  // while the device bakes
+  const cudaError_t done = cudaStreamSynchronize(0);
+  cudaFree(cells);
+  if (baked || done != cudaSuccess)
+    return fail(PSC_ERR_CUDA, "noise bake failed: %s", cudaGetErrorString(done));
+  c->have_base = c->have_detail = c->have_curl = true;
   rc = psc_upload_noise(c, PSC_NOISE_BLUE, blue.data(), blue.size());
   if (rc) return rc;
   c->store_form = -1;

@@ -260,8 +260,10 @@ int launch_composite(const float4* l, const float4* t, float4* hdr, uint32_t n,
                      cudaStream_t stream);
 // RGBA8 volumes of n^3 texels (n a power of two) as 2x2 quads per entry.
 int launch_quads_u8(const uint8_t* src, uint4* quad, uint32_t n, cudaStream_t stream);
-// Noise bakes (noise_bake.cu), synchronous on `stream`.
-int launch_noise_bakes(uint8_t* base, uint8_t* detail, uint8_t* curl, cudaStream_t stream);
+// Noise bakes (noise_bake.cu), queued on `stream`; `cells` is scratch of
+// noise_cells_bytes().
+size_t noise_cells_bytes();
+int launch_noise_bakes(float4* cells, uint8_t* base, uint8_t* detail, uint8_t* curl, cudaStream_t stream);
 // True when a march over these n uniform blocks needs the FAST kernels' full
 // form: a layer of type 7 (Cumulonimbus), a cloud-type grid (its cells may
 // hold any type), Kahan sums, cone light sampling or lightning.  Otherwise
