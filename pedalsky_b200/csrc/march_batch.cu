@@ -67,9 +67,9 @@ __global__ void __launch_bounds__(NT, 768 / NT)
     const uint32_t py = ty * tile_h + (warp / warps_x) * 4u + (lane >> 3);
     if (px < sv.width && py < sv.height) {
       if (FULL && vfull)
-        march_pixel_fast<ST, FILT, true, false, LB>(su, sv, px, py, s_t0, s_t1, s_aux, NT, threadIdx.x);
+        march_pixel_fast<ST, FILT, kFormFull, false, LB>(su, sv, px, py, s_t0, s_t1, s_aux, NT, threadIdx.x);
       else
-        march_pixel_fast<ST, FILT, false, false, LB>(su, sv, px, py, s_t0, s_t1, s_aux, NT, threadIdx.x);
+        march_pixel_fast<ST, FILT, kFormLean, false, LB>(su, sv, px, py, s_t0, s_t1, s_aux, NT, threadIdx.x);
     }
     __syncthreads();  // su, sv and s_tile are rewritten by the next iteration
   }

@@ -1,8 +1,10 @@
 // Single-view FAST march kernel: one thread per ray, CTA tile 16x8 pixels,
 // warps as 8x4 pixel tiles, 8 CTAs per SM for the lean form (64 registers:
 // more resident warps hide more fetch latency than the few spilled values
-// cost) and 7 for the full form (72 registers: its extra paths spill more,
-// and 7 CTAs measured 2.3 % faster on the Cumulonimbus frames).  The per-ray
+// cost) and 7 for the others (72 registers: their extra paths spill more).
+// One 4K frame under a Cumulonimbus layer, 256 + 8 steps: 9.21 ms in the full
+// form, 8.83 in the Cumulonimbus form (8.98 at 8 CTAs per SM, 9.14 at 6), 8.58
+// with its profile's plateau tested first.  The per-ray
 // body is march_fast_body.cuh.
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -16,10 +18,18 @@ constexpr int kTileW = 16;
 constexpr int kTileH = 8;
 constexpr int kThreads = 128;
 
+// The form a march over this uniform block takes: lean without Cumulonimbus
+// layers, a cloud-type grid, Kahan sums, cone sampling and lightning; with
+// Cumulonimbus as the only one of them its own; full otherwise.
+int kernel_form(const MarchUniforms& u) {
+  if (!needs_full_paths(&u, 1)) return kFormLean;
+  return (u.type_grid || u.kahan || u.cone || u.lightning_radius > 0.0f) ? kFormFull : kFormCumulonimbus;
+}
+
 // Shared memory per CTA: the entry/exit distances of each of the view's
 // layers and kAuxWords more words, per thread (dynamic, sized at launch).
-template <int ST, int FILT, bool FULL, int LB>
-__global__ void __launch_bounds__(kThreads, FULL ? 7 : 8) k_march_fast(const __grid_constant__ MarchUniforms u,
+template <int ST, int FILT, int FORM, int LB>
+__global__ void __launch_bounds__(kThreads, FORM == kFormLean ? 8 : 7) k_march_fast(const __grid_constant__ MarchUniforms u,
                                                             const __grid_constant__ ViewDev v) {
   extern __shared__ float s_dyn[];
   const uint32_t nl = u.layer_count;
@@ -30,13 +40,13 @@ __global__ void __launch_bounds__(kThreads, FULL ? 7 : 8) k_march_fast(const __g
   const uint32_t px = blockIdx.x * kTileW + (warp & 1u) * 8u + (lane & 7u);
   const uint32_t py = blockIdx.y * kTileH + (warp >> 1) * 4u + (lane >> 3);
   if (px >= v.width || py >= v.height) return;
-  march_pixel_fast<ST, FILT, FULL, false, LB>(u, v, px, py, s_t0, s_t1, s_aux, kThreads, threadIdx.x);
+  march_pixel_fast<ST, FILT, FORM, false, LB>(u, v, px, py, s_t0, s_t1, s_aux, kThreads, threadIdx.x);
 }
 
 // The instrumented build of the same kernel (psc_count_fetches): every
 // thread counts the fetches its ray issues, and each warp adds its sums to
 // `out` (kTallyKinds 64-bit counters).  Not a timed kernel.
-template <int ST, int FILT, bool FULL>
+template <int ST, int FILT, int FORM>
 __global__ void __launch_bounds__(kThreads) k_march_fast_tally(const __grid_constant__ MarchUniforms u,
                                                                const __grid_constant__ ViewDev v,
                                                                unsigned long long* out) {
@@ -52,7 +62,7 @@ __global__ void __launch_bounds__(kThreads) k_march_fast_tally(const __grid_cons
 #pragma unroll
   for (uint32_t k = 0; k < kTallyKinds; ++k) tc[k] = 0u;
   if (px < v.width && py < v.height)
-    march_pixel_fast<ST, FILT, FULL, true>(u, v, px, py, s_t0, s_t1, s_aux, kThreads, threadIdx.x, tc);
+    march_pixel_fast<ST, FILT, FORM, true>(u, v, px, py, s_t0, s_t1, s_aux, kThreads, threadIdx.x, tc);
 #pragma unroll
   for (uint32_t k = 0; k < kTallyKinds; ++k) {
     const uint32_t sum = __reduce_add_sync(0xffffffffu, tc[k]);
@@ -65,10 +75,11 @@ cudaError_t launch_fast_tally(const MarchUniforms& u, const ViewDev& v, unsigned
                               cudaStream_t s) {
   const dim3 grid((v.width + kTileW - 1) / kTileW, (v.height + kTileH - 1) / kTileH);
   const size_t smem = (2u * u.layer_count + kAuxWords) * kThreads * sizeof(float);
-  if (needs_full_paths(&u, 1))
-    k_march_fast_tally<ST, FILT, true><<<grid, kThreads, smem, s>>>(u, v, out);
-  else
-    k_march_fast_tally<ST, FILT, false><<<grid, kThreads, smem, s>>>(u, v, out);
+  switch (kernel_form(u)) {
+    case kFormLean: k_march_fast_tally<ST, FILT, kFormLean><<<grid, kThreads, smem, s>>>(u, v, out); break;
+    case kFormCumulonimbus: k_march_fast_tally<ST, FILT, kFormCumulonimbus><<<grid, kThreads, smem, s>>>(u, v, out); break;
+    default: k_march_fast_tally<ST, FILT, kFormFull><<<grid, kThreads, smem, s>>>(u, v, out);
+  }
   return cudaGetLastError();
 }
 
@@ -76,10 +87,11 @@ template <int ST, int FILT, int LB = 0>
 cudaError_t launch_fast(const MarchUniforms& u, const ViewDev& v, cudaStream_t s) {
   const dim3 grid((v.width + kTileW - 1) / kTileW, (v.height + kTileH - 1) / kTileH);
   const size_t smem = (2u * u.layer_count + kAuxWords) * kThreads * sizeof(float);
-  if (needs_full_paths(&u, 1))
-    k_march_fast<ST, FILT, true, LB><<<grid, kThreads, smem, s>>>(u, v);
-  else
-    k_march_fast<ST, FILT, false, LB><<<grid, kThreads, smem, s>>>(u, v);
+  switch (kernel_form(u)) {
+    case kFormLean: k_march_fast<ST, FILT, kFormLean, LB><<<grid, kThreads, smem, s>>>(u, v); break;
+    case kFormCumulonimbus: k_march_fast<ST, FILT, kFormCumulonimbus, LB><<<grid, kThreads, smem, s>>>(u, v); break;
+    default: k_march_fast<ST, FILT, kFormFull, LB><<<grid, kThreads, smem, s>>>(u, v);
+  }
   return cudaGetLastError();
 }
 

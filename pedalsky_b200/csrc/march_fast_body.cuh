@@ -35,12 +35,13 @@
 //     LUTs go through the texture unit, as the reference's linear sampler
 //     does; EXACT keeps FP32 weights for them.
 // Octave counts up to 4 are handled here; the host falls back to the plain
-// kernel beyond that.  FULL = false (the lean form) compiles out the paths a
+// kernel beyond that.  The lean form compiles out the paths a
 // common scene does not use: Cumulonimbus (the height-dependent phase of the
 // octaves, the anvil profile of the light march), the cloud-type grid, Kahan
 // sums, cone light sampling and lightning.  The host picks the lean form
-// when none of them is in use (needs_full_paths): the hot loop is shorter and
-// spills less.
+// when none of them is in use, and one between the two for scenes whose only
+// such path is Cumulonimbus (kernel_form): the hot loop is shorter and spills
+// less.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -54,6 +55,8 @@ namespace psc {
 namespace {
 
 constexpr int kMaxOct = 4;
+// Kernel forms (kernel_form): what a form leaves out its scenes do not use.
+constexpr int kFormLean = 0, kFormCumulonimbus = 1, kFormFull = 2;
 
 // atan(a), a in [0, 1]: a * P(a^2), P fitted by iteratively reweighted least
 // squares on Chebyshev nodes (max abs error 3.3e-7 rad in FP32).
@@ -414,7 +417,11 @@ struct NdfTop {
 };
 struct NdfCb {
   float anvil_bias;
-  __device__ __forceinline__ float operator()(float h) const { return ndf_fast(h, 7u, anvil_bias); }
+  // Between its ramps the profile is exactly 1: the base ramp has ended at
+  // 0.05, the middle one falls from 0.5 on and the anvil blends in from 0.65.
+  __device__ __forceinline__ float operator()(float h) const {
+    return (h > 0.0501f && h < 0.4999f) ? 1.0f : ndf_fast(h, 7u, anvil_bias);
+  }
 };
 
 // Base-noise tap of the light march at normalised texture coordinates
@@ -531,10 +538,11 @@ __device__ __forceinline__ float light_march_tex(const MarchUniforms& u, const L
 // Optical depth toward the sun (cloud_march.wgsl:543-578).  `taps`, when
 // given, is lowered to the number of taps fetched where the lean form's
 // light march stops early.
-template <int ST, int FILT, bool FULL = true, int LB = 0>
+template <int ST, int FILT, int FORM = kFormFull, int LB = 0>
 __device__ __forceinline__ float light_od(const MarchUniforms& u, const LayerConst& L, float px,
                                           float py, float pz, float alt, float eff, uint32_t type,
                                           float ux, float uy, float uz, uint32_t* taps = nullptr) {
+  constexpr bool FULL = FORM == kFormFull;  // cone sampling, type grid, Kahan sums
   const float r0 = u.planet_r + alt;
   const float cv = fmaf(ux, u.sun[0], fmaf(uy, u.sun[1], uz * u.sun[2]));
   const float dist = fmaxf((L.top_m - alt) * u.inv_cos_sun, 1.0f);
@@ -566,7 +574,7 @@ __device__ __forceinline__ float light_od(const MarchUniforms& u, const LayerCon
       lr.c1 = cv * lr.ih;
       lr.c2 = s2 * lr.ih;
       lr.c3 = -cv * __fdividef(s2, r0) * lr.ih;
-      if (FULL && type == 7u) return light_march_tex<ST, NdfCb, true, true, FULL, LB>(u, L, lr, NdfCb{L.anvil_bias});
+      if (FORM != kFormLean && type == 7u) return light_march_tex<ST, NdfCb, true, true, FULL, LB>(u, L, lr, NdfCb{L.anvil_bias});
       // heights rise along the light path when cos(up, sun) >= 0 (the cubic's
       // slope stays positive over 20 km), so the first tap bounds them all
       const float t_first = 0.5f * step;
@@ -576,7 +584,7 @@ __device__ __forceinline__ float light_od(const MarchUniforms& u, const LayerCon
         return light_march_tex<ST, NdfTop, false, true, FULL, LB>(u, L, lr, NdfTop{gen.k}, true, taps);
       return light_march_tex<ST, NdfGeneral, false, true, FULL, LB>(u, L, lr, gen, rising, taps);
     }
-    if (FULL && type == 7u) return light_march_tex<ST, NdfCb, true, false, FULL, LB>(u, L, lr, NdfCb{L.anvil_bias});
+    if (FORM != kFormLean && type == 7u) return light_march_tex<ST, NdfCb, true, false, FULL, LB>(u, L, lr, NdfCb{L.anvil_bias});
     return light_march_tex<ST, NdfGeneral, false, false, FULL, LB>(u, L, lr, gen);
   }
   float od = 0.0f, comp = 0.0f;
@@ -715,10 +723,12 @@ static_assert(kTallyKinds == kFetchTallyKinds, "one tally counter per PscFetchCo
 // fetch issued; the timed kernels are built with TALLY = false, where `tc`
 // is unused and the counting compiles away.  LB is the light-march fetch
 // batch (light_march_tex).
-template <int ST, int FILT, bool FULL = true, bool TALLY = false, int LB = 0>
+template <int ST, int FILT, int FORM = kFormFull, bool TALLY = false, int LB = 0>
 __device__ __forceinline__ void march_pixel_fast(const MarchUniforms& u, const ViewDev& v, uint32_t px,
                                                  uint32_t py, float* s_t0, float* s_t1, float* s_aux,
                                                  uint32_t stride, uint32_t slot, uint32_t* tc = nullptr) {
+  constexpr bool FULL = FORM == kFormFull;  // type grid, Kahan sums, cone sampling, lightning
+  constexpr bool CB = FORM != kFormLean;    // Cumulonimbus layers
   if constexpr (TALLY) {
     ++tc[kTallyRays];
     if (v.depth) ++tc[kTallyDepth];
@@ -789,15 +799,15 @@ __device__ __forceinline__ void march_pixel_fast(const MarchUniforms& u, const V
     const float step = __fdividef(segment, (float)u.cloud_steps);
     uint32_t s_begin = 0u, s_end = u.cloud_steps;
     // lean form: the profile test depends on the altitude alone (no type
-    // grid).  The full form keeps every step (the range costs it more than it
-    // saves on the 4K stress frames: 91.6 ms against 88.1 ms).
-    if constexpr (!FULL) {
+    // grid).  The others keep every step (the range costs a Cumulonimbus layer
+    // more than it saves: 8.94 ms a 4K frame against 8.83).
+    if constexpr (!CB) {
       if (!(L.live_lo <= L.live_hi)) continue;  // no step of this layer can pass it
       if (!live_step_range(ray_r0, ray_B, L, u.planet_r, t0, t1, step, jitter, u.cloud_steps, s_begin,
                            s_end))
         continue;
     }
-    const bool cb = FULL && L.cloud_type == 7u && u.phase_mode == PSC_PHASE_APPROX_MIE;
+    const bool cb = CB && L.cloud_type == 7u && u.phase_mode == PSC_PHASE_APPROX_MIE;
     const float cos_theta = FULL ? cos_theta_r : fmaf(dx, u.sun[0], fmaf(dy, u.sun[1], dz * u.sun[2]));
     const float fwd_gain =
         FULL ? fwd_gain_r
@@ -854,7 +864,7 @@ __device__ __forceinline__ void march_pixel_fast(const MarchUniforms& u, const V
         // the lean form has no Cumulonimbus layer, so ndf_mode 0 there means
         // an unknown type, whose profile is 0
         nd = L.ndf_mode ? ndf_eval(NdfCoef{L.ndf_inv_a, L.ndf_b1, L.ndf_inv_w1}, h)
-                        : (FULL ? ndf_fast(h, L.cloud_type, L.anvil_bias) : 0.0f);
+                        : (CB ? ndf_fast(h, L.cloud_type, L.anvil_bias) : 0.0f);
         live = fmaf(nd, 1.000001f, -L.skip_k) * L.density_scale > 1e-3f;
       }
       if (live) {
@@ -908,7 +918,7 @@ __device__ __forceinline__ void march_pixel_fast(const MarchUniforms& u, const V
               tc[kTallyTrans] += trans_fetched ? 1u : 0u;
             }
             uint32_t light_taps_done = (FULL && u.cone) ? 6u : u.light_steps;
-            const float od = light_od<ST, FILT, FULL, LB>(u, L, px3, py3, pz3, alt, eff, type, ux, uy, uz,
+            const float od = light_od<ST, FILT, FORM, LB>(u, L, px3, py3, pz3, alt, eff, type, ux, uy, uz,
                                                           TALLY ? &light_taps_done : nullptr);
             if constexpr (TALLY) tc[kTallyLight] += light_taps_done;
             const float st_r = L.sigma_t[0], st_g = L.sigma_t[1], st_b = L.sigma_t[2];
