@@ -210,9 +210,9 @@ __global__ void __launch_bounds__(kThreads, 5) k_march_plain(const __grid_consta
       const float lsr = fmaxf(density * st_r, 1e-6f), lsg = fmaxf(density * st_g, 1e-6f),
                   lsb = fmaxf(density * st_b, 1e-6f);
       const float smr = expf(-lsr * step), smg = expf(-lsg * step), smb = expf(-lsb * step);
-      const float slr = Tr * ((isr - isr * smr) / lsr);
-      const float slg = Tg * ((isg - isg * smg) / lsg);
-      const float slb = Tb * ((isb - isb * smb) / lsb);
+      const float slr = Tr * div_near(isr - isr * smr, lsr);
+      const float slg = Tg * div_near(isg - isg * smg, lsg);
+      const float slb = Tb * div_near(isb - isb * smb, lsb);
       const float sw = (slr * 0.2126f + slg * 0.7152f) + slb * 0.0722f;
       Lr += slr;
       Lg += slg;

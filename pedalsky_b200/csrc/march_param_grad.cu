@@ -180,7 +180,7 @@ __device__ __forceinline__ DV<A | B> operator*(const DV<A>& x, const DV<B>& y) {
 }
 template <unsigned A, unsigned B>
 __device__ __forceinline__ DV<A | B> operator/(const DV<A>& x, const DV<B>& y) {
-  const float iy = 1.0f / y.v, q = div_by(x.v, y.v, iy);  // no divisor here is 0 or subnormal
+  const float iy = rcp_near(y.v), q = div_by(x.v, y.v, iy);  // no divisor here is 0 or subnormal
   DV<A | B> r;
   r.v = q;
   each<A | B>([&](auto i) {
@@ -206,8 +206,8 @@ template <unsigned M>
 __device__ __forceinline__ DV<M> dlog(const DV<M>& x) { return along(logf(x.v), 1.0f / x.v, x); }
 template <unsigned M>
 __device__ __forceinline__ DV<M> dsqrt(const DV<M>& x) {
-  const float r = sqrtf(fmaxf(x.v, 0.0f));
-  return along(r, r > 0.0f ? 0.5f / r : 0.0f, x);
+  const float r = sqrt_near(fmaxf(x.v, 0.0f));
+  return along(r, r > 1e-19f ? 0.5f * rcp_near(r) : 0.0f, x);
 }
 template <unsigned M>
 __device__ __forceinline__ DV<M> dmax(const DV<M>& x, float m) { return x.v > m ? x : flat<M>(fmaxf(x.v, m)); }

@@ -25,7 +25,7 @@ __device__ __forceinline__ Cover cover_of(const LayerConst& L, float wr) {
   c.eff = clamp01(wr * L.coverage);
   c.ome = 1.0f - c.eff;
   c.den = fmaxf(1.0f - c.ome, 1e-5f);
-  c.inv_den = 1.0f / c.den;
+  c.inv_den = rcp_near(c.den);
   return c;
 }
 
@@ -56,7 +56,8 @@ __device__ __forceinline__ float density_in(const MarchUniforms& u, const LayerC
                                          div_by(ay, u.base_scale, u.inv_base_scale),
                                          div_by(az, u.base_scale, u.inv_base_scale), chk);
   const float lf = clamp01((__fmaf_rn(b.y, 0.625f, __fmul_rn(b.z, 0.25f)) + b.w * 0.125f) + L.lf_bias);
-  const float base_cloud = remapf(b.x, -(1.0f - lf), 1.0f, 0.0f, 1.0f);
+  // remapf(b.x, -(1 - lf), 1, 0, 1)
+  const float a = -(1.0f - lf), base_cloud = 0.0f + div_near(b.x - a, fmaxf(1.0f - a, 1e-5f));
   float cloud = base_cloud * nd;
   cloud = (0.0f + div_by(cloud - cov.ome, cov.den, cov.inv_den)) * cov.eff;
   if (!LIGHT && cloud > 0.0f) {
@@ -70,7 +71,8 @@ __device__ __forceinline__ float density_in(const MarchUniforms& u, const LayerC
                                                div_by(dz, u.detail_scale, inv), chk);
     const float hf = __fmaf_rn(det.x, 0.625f, __fmul_rn(det.y, 0.25f)) + det.z * 0.125f;
     const float dmod = mixf(hf, 1.0f - hf, clamp01(h * 10.0f));
-    cloud = remapf(cloud, dmod * L.layer_detail, 1.0f, 0.0f, 1.0f);
+    const float lo = dmod * L.layer_detail;
+    cloud = 0.0f + div_near(cloud - lo, fmaxf(1.0f - lo, 1e-5f));  // remapf(cloud, lo, 1, 0, 1)
   }
   return clamp01(cloud) * L.density_scale;
 }
@@ -107,9 +109,9 @@ __device__ __forceinline__ float altitude_from_entry(const MarchUniforms& u, flo
   // contractions written out: the last bit of the altitude moves the noise
   // coordinates, and left to the compiler it follows the code around the call
   const float yy = py + u.planet_r;
-  const float len = sqrtf(__fmaf_rn(pz, pz, __fmaf_rn(px, px, __fmul_rn(yy, yy))));
+  const float len = sqrt_near(__fmaf_rn(pz, pz, __fmaf_rn(px, px, __fmul_rn(yy, yy))));
   const float num = __fmaf_rn(t, t, 2.0f * t * r0 * cos_view);
-  return h0 + num / (fmaxf(r0, 1.0f) + len);
+  return h0 + div_near(num, fmaxf(r0, 1.0f) + len);
 }
 
 template <int ST, int FILT>
@@ -117,7 +119,7 @@ __device__ float march_to_light(const MarchUniforms& u, const LayerConst& L, flo
                                 float pz, float alt, const Cover& cov, uint32_t type, int* chk) {
   const float sx = u.sun[0], sy = u.sun[1], sz = u.sun[2];
   const float r0 = u.planet_r + alt;
-  const float inv = 1.0f / fmaxf(r0, 1.0f);
+  const float inv = rcp_near(fmaxf(r0, 1.0f));
   const float cv = ((px * inv) * sx + ((py + u.planet_r) * inv) * sy) + (pz * inv) * sz;
   const float cos_sun = fmaxf(sy, 0.05f);
   const float dist = fmaxf(div_by(L.top_m - alt, cos_sun, u.inv_cos_sun), 1.0f);
@@ -148,7 +150,7 @@ __device__ float march_to_light(const MarchUniforms& u, const LayerConst& L, flo
     od += density_light_at<ST, FILT>(u, L, qx, qy, qz, a, cov, type, chk) * step * 3.0f;
     return od;
   }
-  const float step = dist / (float)u.light_steps;
+  const float step = div_near(dist, (float)u.light_steps);
 #pragma unroll 1
   for (uint32_t i = 0; i < u.light_steps; ++i) {
     const float t = ((float)i + 0.5f) * step;
@@ -183,36 +185,36 @@ __device__ __forceinline__ SunSky sun_and_sky_at(const MarchUniforms& u, float p
   SunSky out;
   const float R = u.planet_r;
   const float ay = py + R;
-  const float len = sqrtf(__fmaf_rn(pz, pz, __fmaf_rn(px, px, __fmul_rn(ay, ay))));
+  const float len = sqrt_near(__fmaf_rn(pz, pz, __fmaf_rn(px, px, __fmul_rn(ay, ay))));
   const float r = fmaxf(len, R + 1.0f);
-  const float inv_len = 1.0f / len, inv_r = r == len ? inv_len : 1.0f / r;
+  const float inv_len = rcp_near(len), inv_r = r == len ? inv_len : rcp_near(r);
   const float mu = clampf((div_by(px, r, inv_r) * u.sun[0] + div_by(ay, r, inv_r) * u.sun[1]) +
                               div_by(pz, r, inv_r) * u.sun[2], -1.0f, 1.0f);
   const float ratio = div_by(R, r, inv_r);
-  const float sin_h = -sqrtf(fmaxf(1.0f - ratio * ratio, 0.0f));
+  const float sin_h = -sqrt_near(fmaxf(1.0f - ratio * ratio, 0.0f));
   if (mu <= sin_h) {
     out.sun = make_float3(0.0f, 0.0f, 0.0f);
   } else {
     const float ht = u.atmo_top;
-    const float rho = sqrtf(fmaxf(r * r - R * R, 0.0f));
+    const float rho = sqrt_near(fmaxf(r * r - R * R, 0.0f));
     const float disc = r * r * (mu * mu - 1.0f) + ht * ht;
-    const float d = fmaxf(-r * mu + sqrtf(fmaxf(disc, 0.0f)), 0.0f);
+    const float d = fmaxf(-r * mu + sqrt_near(fmaxf(disc, 0.0f)), 0.0f);
     const float d_min = ht - r, d_max = rho + bh;
-    const float xm = clamp01((d - d_min) / fmaxf(d_max - d_min, 1.0f));
+    const float xm = clamp01(div_near(d - d_min, fmaxf(d_max - d_min, 1.0f)));
     const float xr = div_by(rho, fmaxf(bh, 1.0f), inv_bh);
     const float4 t = lut2d(u.lut_trans, 256, 64, xm, xr, chk, kChkTrans);
     out.sun = make_float3(t.x, t.y, t.z);
   }
   const float ux = div_by(px, len, inv_len), uy = div_by(ay, len, inv_len), uz = div_by(pz, len, inv_len);
-  const float vza = atan2f(sqrtf(ux * ux + uz * uz), uy);
+  const float vza = atan2f(sqrt_near(ux * ux + uz * uz), uy);
   const float sin_z = clamp01(div_by(R, len, inv_len));
   const float zha = kPi - asinf(sin_z);
   float vv;
   if (vza < zha) {
-    vv = sqrtf(clamp01(vza / fmaxf(zha, 1e-6f))) * 0.5f;
+    vv = sqrt_near(clamp01(div_near(vza, fmaxf(zha, 1e-6f)))) * 0.5f;
   } else {
     const float br = fmaxf(kPi - zha, 1e-6f);
-    vv = 0.5f + sqrtf(clamp01((vza - zha) / br)) * 0.5f;
+    vv = 0.5f + sqrt_near(clamp01(div_near(vza - zha, br))) * 0.5f;
   }
   const float vaz = atan2f(ux, uz);
   float du = div_by(vaz - sun_az, 2.0f * kPi, 1.0f / (2.0f * kPi));
