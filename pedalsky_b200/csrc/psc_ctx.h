@@ -102,6 +102,7 @@ struct psc_ctx {
   // largest grid seen; GridDev::nonfinite lies behind the quads
   float4* d_grid_quads = nullptr;
   float4* d_grid_grads = nullptr;
+  cudaEvent_t grid_done = nullptr;  // the last grid call's end: the next one, on whatever stream, waits for it
   size_t grid_quads_cap = 0, grid_grads_cap = 0;  // entries
   uint32_t* d_btiles = nullptr;
   uint32_t* d_bcounter = nullptr;

@@ -1568,6 +1568,8 @@ int psc_destroy(psc_ctx* c) {
   dfree(c->d_check);
   dfree(c->d_grid_quads);
   dfree(c->d_grid_grads);
+  if (c->grid_done) cudaEventDestroy(c->grid_done);
+  c->grid_done = nullptr;
   for (auto& tv : c->taa) free_taa_view(tv);
   dfree(c->d_blue);
   dfree(c->d_weather);
@@ -2504,10 +2506,40 @@ int prepare_grid(psc_ctx* c, const PscDensityGrid* g, const PscView* v, bool adj
   return PSC_OK;
 }
 
+bool capturing(cudaStream_t s) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return st != cudaStreamCaptureStatusNone;
+}
+
+// Allocations made while a stream is captured (a first grid call) are the
+// context's own and no part of the graph.
+struct RelaxedCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+// The grid calls of a context share its quads: each marks its end on its
+// stream, and the next one waits for that.  Calls that are being captured are
+// ordered by their graph.
+int grid_call_done(psc_ctx* c, cudaStream_t s) {
+  if (capturing(s)) return PSC_OK;
+  if (!c->grid_done)
+    PSC_CUDA(cudaEventCreateWithFlags(&c->grid_done, cudaEventDisableTiming), "grid event");
+  PSC_CUDA(cudaEventRecord(c->grid_done, s), "grid event record");
+  return PSC_OK;
+}
+
 // The grid values as (x, z) corner quads (GridDev::quads) on `s`, and for the
 // adjoint a zeroed gradient of the same form (GridDev::grads).
 int stage_grid_layout(psc_ctx* c, psc::GridDev& gd, bool adjoint, cudaStream_t s) {
   const size_t nq = (size_t)gd.plane * (gd.ny + 4u);
+  RelaxedCapture relaxed;
+  if (c->grid_done && !capturing(s)) PSC_CUDA(cudaStreamWaitEvent(s, c->grid_done, 0), "grid event wait");
   if (c->grid_quads_cap < nq) {
     dfree(c->d_grid_quads);
     c->grid_quads_cap = 0;
@@ -2543,7 +2575,7 @@ int psc_render_grid(psc_ctx* c, const PscDensityGrid* g, const PscView* v, void*
   rc = psc::launch_grid_march(u, vd, gd, false, static_cast<cudaStream_t>(stream));
   if (rc) return fail(rc, "grid march launch failed: %s", cudaGetErrorString(cudaGetLastError()));
   ++c->launches;
-  return PSC_OK;
+  return grid_call_done(c, static_cast<cudaStream_t>(stream));
 }
 
 int psc_adjoint(psc_ctx* c, const PscDensityGrid* g, const PscView* v, const float* background,
@@ -2569,7 +2601,7 @@ int psc_adjoint(psc_ctx* c, const PscDensityGrid* g, const PscView* v, const flo
   rc = psc::launch_grid_fold(gd.grads, grad_values, gd.nx, gd.ny, gd.nz, s);
   if (rc) return fail(rc, "gradient fold launch failed: %s", cudaGetErrorString(cudaGetLastError()));
   ++c->launches;
-  return PSC_OK;
+  return grid_call_done(c, s);
 }
 
 int psc_layer_gradient(psc_ctx* c, const PscDensityGrid* g, const PscView* v, const float* background,
@@ -2597,7 +2629,7 @@ int psc_layer_gradient(psc_ctx* c, const PscDensityGrid* g, const PscView* v, co
   rc = psc::launch_grid_layer_grad(u, vd, gd, grad_base_top, static_cast<cudaStream_t>(stream));
   if (rc) return fail(rc, "layer-gradient launch failed: %s", cudaGetErrorString(cudaGetLastError()));
   ++c->launches;
-  return PSC_OK;
+  return grid_call_done(c, static_cast<cudaStream_t>(stream));
 }
 
 int psc_layer_param_gradient(psc_ctx* c, const PscView* v, uint32_t layer, const float* background,
