@@ -20,10 +20,14 @@ constexpr int kThreads = 128;
 
 // The form a march over this uniform block takes: lean without Cumulonimbus
 // layers, a cloud-type grid, Kahan sums, cone sampling and lightning; with
-// Cumulonimbus as the only one of them its own; full otherwise.
-int kernel_form(const MarchUniforms& u) {
+// Cumulonimbus as the only one of them its own, in its form for few CTAs up to
+// one per SM (110 CTAs are slower with the plateau, 255 even, 510 faster); full
+// otherwise.
+constexpr uint32_t kFewCtas = 148;
+int kernel_form(const MarchUniforms& u, const dim3& grid) {
   if (!needs_full_paths(&u, 1)) return kFormLean;
-  return (u.type_grid || u.kahan || u.cone || u.lightning_radius > 0.0f) ? kFormFull : kFormCumulonimbus;
+  if (u.type_grid || u.kahan || u.cone || u.lightning_radius > 0.0f) return kFormFull;
+  return grid.x * grid.y <= kFewCtas ? kFormCumulonimbusFew : kFormCumulonimbus;
 }
 
 // Shared memory per CTA: the entry/exit distances of each of the view's
@@ -75,8 +79,9 @@ cudaError_t launch_fast_tally(const MarchUniforms& u, const ViewDev& v, unsigned
                               cudaStream_t s) {
   const dim3 grid((v.width + kTileW - 1) / kTileW, (v.height + kTileH - 1) / kTileH);
   const size_t smem = (2u * u.layer_count + kAuxWords) * kThreads * sizeof(float);
-  switch (kernel_form(u)) {
+  switch (kernel_form(u, grid)) {
     case kFormLean: k_march_fast_tally<ST, FILT, kFormLean><<<grid, kThreads, smem, s>>>(u, v, out); break;
+    case kFormCumulonimbusFew:  // the same fetches
     case kFormCumulonimbus: k_march_fast_tally<ST, FILT, kFormCumulonimbus><<<grid, kThreads, smem, s>>>(u, v, out); break;
     default: k_march_fast_tally<ST, FILT, kFormFull><<<grid, kThreads, smem, s>>>(u, v, out);
   }
@@ -87,8 +92,11 @@ template <int ST, int FILT, int LB = 0>
 cudaError_t launch_fast(const MarchUniforms& u, const ViewDev& v, cudaStream_t s) {
   const dim3 grid((v.width + kTileW - 1) / kTileW, (v.height + kTileH - 1) / kTileH);
   const size_t smem = (2u * u.layer_count + kAuxWords) * kThreads * sizeof(float);
-  switch (kernel_form(u)) {
+  switch (kernel_form(u, grid)) {
     case kFormLean: k_march_fast<ST, FILT, kFormLean, LB><<<grid, kThreads, smem, s>>>(u, v); break;
+    case kFormCumulonimbusFew:
+      k_march_fast<ST, FILT, kFormCumulonimbusFew, LB><<<grid, kThreads, smem, s>>>(u, v);
+      break;
     case kFormCumulonimbus: k_march_fast<ST, FILT, kFormCumulonimbus, LB><<<grid, kThreads, smem, s>>>(u, v); break;
     default: k_march_fast<ST, FILT, kFormFull, LB><<<grid, kThreads, smem, s>>>(u, v);
   }

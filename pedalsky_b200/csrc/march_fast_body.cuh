@@ -56,7 +56,8 @@ namespace {
 
 constexpr int kMaxOct = 4;
 // Kernel forms (kernel_form): what a form leaves out its scenes do not use.
-constexpr int kFormLean = 0, kFormCumulonimbus = 1, kFormFull = 2;
+// kFormCumulonimbusFew is kFormCumulonimbus for launches of few CTAs (NdfCb).
+constexpr int kFormLean = 0, kFormCumulonimbus = 1, kFormFull = 2, kFormCumulonimbusFew = 3;
 
 // atan(a), a in [0, 1]: a * P(a^2), P fitted by iteratively reweighted least
 // squares on Chebyshev nodes (max abs error 3.3e-7 rad in FP32).
@@ -415,12 +416,18 @@ struct NdfTop {
   NdfCoef k;
   __device__ __forceinline__ float operator()(float h) const { return ssr_b(k.inv_w1, k.b1, h); }
 };
+// PLATEAU: between its ramps the profile is exactly 1 (the base ramp has ended
+// at 0.05, the middle one falls from 0.5 on and the anvil blends in from 0.65),
+// and its ramps are not evaluated there.  That saves instructions and puts a
+// branch in front of every tap, so it pays where warps fill the schedulers and
+// costs where a launch is one ray's chain of latencies: 3840x2160 8.83 -> 8.58
+// ms, 960x540 998 -> 975 us, but 147x83 203 -> 209 us and 96x54 551 -> 560 us.
+template <bool PLATEAU>
 struct NdfCb {
   float anvil_bias;
-  // Between its ramps the profile is exactly 1: the base ramp has ended at
-  // 0.05, the middle one falls from 0.5 on and the anvil blends in from 0.65.
   __device__ __forceinline__ float operator()(float h) const {
-    return (h > 0.0501f && h < 0.4999f) ? 1.0f : ndf_fast(h, 7u, anvil_bias);
+    if (PLATEAU && h > 0.0501f && h < 0.4999f) return 1.0f;
+    return ndf_fast(h, 7u, anvil_bias);
   }
 };
 
@@ -543,6 +550,7 @@ __device__ __forceinline__ float light_od(const MarchUniforms& u, const LayerCon
                                           float py, float pz, float alt, float eff, uint32_t type,
                                           float ux, float uy, float uz, uint32_t* taps = nullptr) {
   constexpr bool FULL = FORM == kFormFull;  // cone sampling, type grid, Kahan sums
+  using NdfCbF = NdfCb<FORM != kFormCumulonimbusFew>;
   const float r0 = u.planet_r + alt;
   const float cv = fmaf(ux, u.sun[0], fmaf(uy, u.sun[1], uz * u.sun[2]));
   const float dist = fmaxf((L.top_m - alt) * u.inv_cos_sun, 1.0f);
@@ -574,7 +582,7 @@ __device__ __forceinline__ float light_od(const MarchUniforms& u, const LayerCon
       lr.c1 = cv * lr.ih;
       lr.c2 = s2 * lr.ih;
       lr.c3 = -cv * __fdividef(s2, r0) * lr.ih;
-      if (FORM != kFormLean && type == 7u) return light_march_tex<ST, NdfCb, true, true, FULL, LB>(u, L, lr, NdfCb{L.anvil_bias});
+      if (FORM != kFormLean && type == 7u) return light_march_tex<ST, NdfCbF, true, true, FULL, LB>(u, L, lr, NdfCbF{L.anvil_bias});
       // heights rise along the light path when cos(up, sun) >= 0 (the cubic's
       // slope stays positive over 20 km), so the first tap bounds them all
       const float t_first = 0.5f * step;
@@ -584,7 +592,7 @@ __device__ __forceinline__ float light_od(const MarchUniforms& u, const LayerCon
         return light_march_tex<ST, NdfTop, false, true, FULL, LB>(u, L, lr, NdfTop{gen.k}, true, taps);
       return light_march_tex<ST, NdfGeneral, false, true, FULL, LB>(u, L, lr, gen, rising, taps);
     }
-    if (FORM != kFormLean && type == 7u) return light_march_tex<ST, NdfCb, true, false, FULL, LB>(u, L, lr, NdfCb{L.anvil_bias});
+    if (FORM != kFormLean && type == 7u) return light_march_tex<ST, NdfCbF, true, false, FULL, LB>(u, L, lr, NdfCbF{L.anvil_bias});
     return light_march_tex<ST, NdfGeneral, false, false, FULL, LB>(u, L, lr, gen);
   }
   float od = 0.0f, comp = 0.0f;
