@@ -625,7 +625,16 @@ typedef struct PscDensityGrid {
 
 /* Forward march of the grid form for each view (device `values`);
  * outputs as psc_render (luminance, transmittance, optional composite).
- * Needs the frame, blue noise and the transmittance and sky-view LUTs. */
+ * Needs the frame, blue noise and the transmittance and sky-view LUTs.
+ *
+ * Grid calls (this one, psc_adjoint, psc_layer_gradient) of one context may
+ * be queued on any streams: they share scratch that grows to the largest grid
+ * and run one after the other.  A call on a capturing stream takes scratch of
+ * its own (16 bytes per cell, 32 for the adjoint), which its graph keeps until
+ * the graph and its executables are destroyed, so a graph may be replayed
+ * beside other grid calls and other graphs; two launches of the same captured
+ * call must not overlap.  As with any captured call, the context and the
+ * inputs it held must still be there. */
 int psc_render_grid(psc_ctx* ctx, const PscDensityGrid* grid, const PscView* view, void* stream);
 
 /* Gradient of an image loss with respect to the grid values and

@@ -5,12 +5,30 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
 #include <string>
 #include <vector>
 
 #include "../../include/psclouds.h"
 #include "psc_internal.h"
+
+namespace psc {
+namespace host {
+
+// Scratch of one captured grid call.  The graph it is captured into holds a
+// reference (a CUDA user object, so its copies and executables count too) and
+// the context one: no other call gets the memory while a graph can replay
+// into it, and the context takes it back or frees it afterwards.
+struct GraphScratch {
+  void* p = nullptr;
+  size_t bytes = 0;
+  std::atomic<uint32_t> refs{1};  // 1: the context alone
+  GraphScratch* next = nullptr;
+};
+
+}  // namespace host
+}  // namespace psc
 
 struct psc_ctx {
   int device = 0;
@@ -103,6 +121,7 @@ struct psc_ctx {
   float4* d_grid_quads = nullptr;
   float4* d_grid_grads = nullptr;
   cudaEvent_t grid_done = nullptr;  // the last grid call's end: the next one, on whatever stream, waits for it
+  psc::host::GraphScratch* graph_scratch = nullptr;  // of captured grid calls
   size_t grid_quads_cap = 0, grid_grads_cap = 0;  // entries
   uint32_t* d_btiles = nullptr;
   uint32_t* d_bcounter = nullptr;

@@ -14,6 +14,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <new>
 #include <string>
 #include <vector>
 
@@ -71,6 +72,7 @@ int ensure_device(psc_ctx* c) {
 using psc::host::cuda_fail;
 using psc::host::ensure_device;
 using psc::host::fail;
+using psc::host::GraphScratch;
 
 namespace {
 
@@ -1570,6 +1572,11 @@ int psc_destroy(psc_ctx* c) {
   dfree(c->d_grid_grads);
   if (c->grid_done) cudaEventDestroy(c->grid_done);
   c->grid_done = nullptr;
+  while (GraphScratch* g = c->graph_scratch) {  // a graph still there must not be launched any more
+    c->graph_scratch = g->next;
+    cudaFree(g->p);
+    if (g->refs.fetch_sub(1, std::memory_order_acq_rel) == 1) delete g;
+  }
   for (auto& tv : c->taa) free_taa_view(tv);
   dfree(c->d_blue);
   dfree(c->d_weather);
@@ -2515,17 +2522,77 @@ bool capturing(cudaStream_t s) {
   return st != cudaStreamCaptureStatusNone;
 }
 
-// Allocations made while a stream is captured (a first grid call) are the
-// context's own and no part of the graph.
+// Allocations made while a stream is captured are no part of the graph.
 struct RelaxedCapture {
   cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
   RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
   ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
 };
 
+void drop_graph_scratch(void* p) {
+  auto* const g = static_cast<GraphScratch*>(p);
+  if (g->refs.fetch_sub(1, std::memory_order_acq_rel) == 1) delete g;
+}
+
+// Frees the scratch whose graphs are gone, but one of at least `bytes` and at
+// most twice that (0: keeps none), which is returned.
+GraphScratch* idle_graph_scratch(psc_ctx* c, size_t bytes) {
+  GraphScratch* keep = nullptr;
+  for (GraphScratch** at = &c->graph_scratch; *at;) {
+    GraphScratch* const g = *at;
+    if (g->refs.load(std::memory_order_acquire) == 1) {
+      if (keep || g->bytes < bytes || g->bytes / 2 > bytes) {
+        *at = g->next;
+        cudaFree(g->p);
+        delete g;
+        continue;
+      }
+      keep = g;
+    }
+    at = &g->next;
+  }
+  return keep;
+}
+
+// `bytes` of scratch for a call captured on `s`, the graph's own for as long
+// as it lives.
+int graph_scratch(psc_ctx* c, size_t bytes, cudaStream_t s, void** out) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  cudaGraph_t graph = nullptr;
+  PSC_CUDA(cudaStreamGetCaptureInfo(s, &st, nullptr, &graph), "capture info");
+  if (st != cudaStreamCaptureStatusActive) return fail(PSC_ERR_CUDA, "the stream's capture is invalid");
+  GraphScratch* g = idle_graph_scratch(c, bytes);
+  if (!g) {
+    g = new (std::nothrow) GraphScratch;
+    if (!g) return fail(PSC_ERR_CUDA, "out of host memory");
+    const cudaError_t e = cudaMalloc(&g->p, bytes);
+    if (e != cudaSuccess) {
+      delete g;
+      return cuda_fail(e, "cudaMalloc captured grid scratch");
+    }
+    g->bytes = bytes;
+    g->next = c->graph_scratch;
+    c->graph_scratch = g;
+  }
+  g->refs.fetch_add(1, std::memory_order_relaxed);
+  cudaUserObject_t held = nullptr;
+  cudaError_t e = cudaUserObjectCreate(&held, g, drop_graph_scratch, 1, cudaUserObjectNoDestructorSync);
+  if (e != cudaSuccess) {
+    drop_graph_scratch(g);
+    return cuda_fail(e, "grid scratch user object");
+  }
+  e = cudaGraphRetainUserObject(graph, held, 1, cudaGraphUserObjectMove);
+  if (e != cudaSuccess) {
+    cudaUserObjectRelease(held, 1);
+    return cuda_fail(e, "grid scratch of the graph");
+  }
+  *out = g->p;
+  return PSC_OK;
+}
+
 // The grid calls of a context share its quads: each marks its end on its
-// stream, and the next one waits for that.  Calls that are being captured are
-// ordered by their graph.
+// stream, and the next one waits for that.  A captured call has its graph's
+// own and needs neither.
 int grid_call_done(psc_ctx* c, cudaStream_t s) {
   if (capturing(s)) return PSC_OK;
   if (!c->grid_done)
@@ -2539,23 +2606,39 @@ int grid_call_done(psc_ctx* c, cudaStream_t s) {
 int stage_grid_layout(psc_ctx* c, psc::GridDev& gd, bool adjoint, cudaStream_t s) {
   const size_t nq = (size_t)gd.plane * (gd.ny + 4u);
   RelaxedCapture relaxed;
-  if (c->grid_done && !capturing(s)) PSC_CUDA(cudaStreamWaitEvent(s, c->grid_done, 0), "grid event wait");
-  if (c->grid_quads_cap < nq) {
-    dfree(c->d_grid_quads);
-    c->grid_quads_cap = 0;
-    PSC_CUDA(cudaMalloc(&c->d_grid_quads, (nq + 1u) * sizeof(float4)), "cudaMalloc grid quads");  // + the flag
-    c->grid_quads_cap = nq;
+  float4 *quads = nullptr, *grads = nullptr;
+  uint32_t* nonfinite = nullptr;  // behind the quads
+  if (capturing(s)) {
+    void* p = nullptr;
+    const int rc = graph_scratch(c, (nq * (adjoint ? 2u : 1u) + 1u) * sizeof(float4), s, &p);
+    if (rc) return rc;
+    quads = static_cast<float4*>(p);
+    nonfinite = reinterpret_cast<uint32_t*>(quads + nq);
+    grads = adjoint ? quads + nq + 1u : nullptr;
+  } else {
+    idle_graph_scratch(c, 0);
+    if (c->grid_done) PSC_CUDA(cudaStreamWaitEvent(s, c->grid_done, 0), "grid event wait");
+    if (c->grid_quads_cap < nq) {
+      dfree(c->d_grid_quads);
+      c->grid_quads_cap = 0;
+      PSC_CUDA(cudaMalloc(&c->d_grid_quads, (nq + 1u) * sizeof(float4)), "cudaMalloc grid quads");
+      c->grid_quads_cap = nq;
+    }
+    quads = c->d_grid_quads;
+    nonfinite = reinterpret_cast<uint32_t*>(quads + c->grid_quads_cap);
+    if (adjoint) {
+      const int rc = grow(&c->d_grid_grads, &c->grid_grads_cap, nq, "cudaMalloc gradient quads");
+      if (rc) return rc;
+      grads = c->d_grid_grads;
+    }
   }
-  uint32_t* const nonfinite = reinterpret_cast<uint32_t*>(c->d_grid_quads + c->grid_quads_cap);
-  if (psc::launch_grid_quads(gd.values, c->d_grid_quads, nonfinite, gd.nx, gd.ny, gd.nz, s))
+  if (psc::launch_grid_quads(gd.values, quads, nonfinite, gd.nx, gd.ny, gd.nz, s))
     return fail(PSC_ERR_CUDA, "grid quad launch failed: %s", cudaGetErrorString(cudaGetLastError()));
-  gd.quads = c->d_grid_quads;
+  gd.quads = quads;
   gd.nonfinite = nonfinite;
   if (adjoint) {
-    int rc = grow(&c->d_grid_grads, &c->grid_grads_cap, nq, "cudaMalloc gradient quads");
-    if (rc) return rc;
-    PSC_CUDA(cudaMemsetAsync(c->d_grid_grads, 0, nq * sizeof(float4), s), "gradient quad reset");
-    gd.grads = c->d_grid_grads;
+    PSC_CUDA(cudaMemsetAsync(grads, 0, nq * sizeof(float4), s), "gradient quad reset");
+    gd.grads = grads;
   }
   return PSC_OK;
 }
