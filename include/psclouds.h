@@ -613,8 +613,8 @@ typedef struct PscDensityGrid {
   uint32_t nx, ny, nz;          /* cells along world x (east), altitude, world z (south) */
   uint32_t checkpoint_every;    /* psc_adjoint, psc_layer_gradient: 1..32, at most
                                    PSC_GRID_MAX_CHECKPOINTS intervals; checked, and without effect
-                                   on the result (the reverse sweep walks the optical depth back
-                                   exactly and needs no checkpoints) */
+                                   on the result (the reverse sweep takes the optical depth back
+                                   step by step and needs no checkpoints) */
   float min_x_m, min_z_m;       /* world x / z of the grid's low corner */
   float size_x_m, size_z_m;     /* horizontal extent (altitude extent: layer 0 base..top) */
   float density_scale;          /* multiplies every value */
