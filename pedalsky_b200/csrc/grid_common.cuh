@@ -25,14 +25,15 @@ __device__ __forceinline__ GridPos grid_pos(const GridDev& g, float x, float alt
 
 // The eight corners around a point: the index of its quad in the stored
 // arrays (GridDev::quads, grads) and the weights of the upper corners.  Each
-// coordinate is held to [-2, n]; the arrays hold two layers of zeros before
-// the first cell of every axis and two behind the last, so a point outside
-// reads zeros without a bounds test.  WIDE: arrays too large for floor_bits
-// or a 32-bit index (grid_wide).
+// coordinate is held to [-2, n].  The narrow arrays hold two layers of zeros
+// before the first cell of every axis and two behind the last, so a point
+// outside reads zeros without a bounds test; in the wide ones (GridDev::wide)
+// a row of corners is read where the grid has it.
 template <bool WIDE>
 struct Cell {
   std::conditional_t<WIDE, size_t, uint32_t> i;  // quad of the lower y row; the upper is g.plane further on
   float wx, wy, wz;
+  bool lo, hi;  // WIDE: the array holds the lower, the upper y row
 };
 
 template <bool WIDE>
@@ -42,7 +43,11 @@ __device__ __forceinline__ Cell<WIDE> grid_cell(const GridDev& g, const GridPos&
   Cell<WIDE> c;
   if constexpr (WIDE) {
     const float fx = floorf(x), fy = floorf(y), fz = floorf(z);
-    c.i = (size_t)((int64_t)fy + 2) * g.plane + (size_t)((int64_t)fz + 2) * g.row + (size_t)((int64_t)fx + 2);
+    const int64_t ix = (int64_t)fx, iy = (int64_t)fy, iz = (int64_t)fz;
+    const bool in = (uint64_t)(ix + 1) <= g.nx && (uint64_t)(iz + 1) <= g.nz;
+    c.lo = in && (uint64_t)iy < g.ny;
+    c.hi = in && (uint64_t)(iy + 1) < g.ny;
+    c.i = (size_t)iy * g.plane + (size_t)(iz + 1) * g.row + (size_t)(ix + 1);
     c.wx = x - fx;
     c.wy = y - fy;
     c.wz = z - fz;
@@ -50,6 +55,7 @@ __device__ __forceinline__ Cell<WIDE> grid_cell(const GridDev& g, const GridPos&
     // floor_bits counts from 0x4B400000; g.origin takes that and the two
     // layers before the first cell off all three axes at once (mod 2^32)
     const FloorBits fx = floor_bits(x), fy = floor_bits(y), fz = floor_bits(z);
+    c.lo = c.hi = true;
     c.i = fy.i * (uint32_t)g.plane + fz.i * g.row + (fx.i - g.origin);
     c.wx = x - fx.f;
     c.wy = y - fy.f;
@@ -58,9 +64,15 @@ __device__ __forceinline__ Cell<WIDE> grid_cell(const GridDev& g, const GridPos&
   return c;
 }
 
-// floor_bits counts cells exactly up to 2^22; the narrow kernels index in 32 bits.
-inline bool grid_wide(const GridDev& g) {
-  return g.nx >= (1u << 21) || g.ny >= (1u << 21) || g.nz >= (1u << 21) || g.plane * (g.ny + 4ull) >= (1ull << 31);
+// The cell's quads at its lower and upper y.
+struct Rows {
+  float4 a, b;
+};
+template <bool WIDE>
+__device__ __forceinline__ Rows grid_rows(const GridDev& g, const Cell<WIDE>& c) {
+  const float4 none = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  return {!WIDE || c.lo ? __ldg(g.quads + c.i) : none,
+          !WIDE || c.hi ? __ldg(g.quads + (c.i + (decltype(c.i))g.plane)) : none};
 }
 
 // Whether a point has a corner inside the grid.  One without has grid value
@@ -75,7 +87,7 @@ template <bool WIDE>
 __device__ __forceinline__ float grid_fetch(const GridDev& g, const Cell<WIDE>& c) {
   const float wx0 = 1.0f - c.wx, wy0 = 1.0f - c.wy;
   const float2 x0 = make_float2(wx0, wx0), x1 = make_float2(c.wx, c.wx), wz = make_float2(1.0f - c.wz, c.wz);
-  const float4 a = __ldg(g.quads + c.i), b = __ldg(g.quads + (c.i + (decltype(c.i))g.plane));
+  const auto [a, b] = grid_rows<WIDE>(g, c);
   const float2 ha = fma2(x1, make_float2(a.z, a.w), mul2(x0, make_float2(a.x, a.y)));
   const float2 hb = fma2(x1, make_float2(b.z, b.w), mul2(x0, make_float2(b.x, b.y)));
   const float2 v = fma2(mul2(make_float2(c.wy, c.wy), wz), hb, mul2(mul2(make_float2(wy0, wy0), wz), ha));

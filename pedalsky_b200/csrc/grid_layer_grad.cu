@@ -90,7 +90,7 @@ __device__ __forceinline__ D2 alt_from_d(const MarchUniforms& u, D2 qx, D2 qy, D
 // value and its derivatives are 0.
 template <bool WIDE>
 __device__ __forceinline__ bool cell_filled(const GridDev& g, const Cell<WIDE>& c) {
-  const float4 a = __ldg(g.quads + c.i), b = __ldg(g.quads + (c.i + (decltype(c.i))g.plane));
+  const auto [a, b] = grid_rows<WIDE>(g, c);
   const uint32_t bits = __float_as_uint(a.x) | __float_as_uint(a.y) | __float_as_uint(a.z) | __float_as_uint(a.w) |
                         __float_as_uint(b.x) | __float_as_uint(b.y) | __float_as_uint(b.z) | __float_as_uint(b.w);
   return (bits << 1) != 0u;  // -0 is empty too
@@ -103,7 +103,7 @@ struct GridSlopes {
 template <bool WIDE>
 __device__ __forceinline__ GridSlopes grid_fetch_slopes(const GridDev& g, const GridPos& p) {
   const Cell<WIDE> c = grid_cell<WIDE>(g, p);
-  const float4 a = __ldg(g.quads + c.i), b = __ldg(g.quads + (c.i + (decltype(c.i))g.plane));
+  const auto [a, b] = grid_rows<WIDE>(g, c);
   // the quad's lanes are (z, x): 00, 10, 01, 11
   const float a0 = fmaf(c.wz, a.y - a.x, a.x), a1 = fmaf(c.wz, a.w - a.z, a.z);
   const float b0 = fmaf(c.wz, b.y - b.x, b.x), b1 = fmaf(c.wz, b.w - b.z, b.z);
@@ -408,7 +408,7 @@ int launch_grid_layer_grad(const MarchUniforms& u, const ViewDev& v, const GridD
   if (!g.quads) return PSC_ERR_INVALID_ARGUMENT;
   if (u.octaves == 0 || u.octaves > (uint32_t)kMaxOct) return PSC_ERR_UNSUPPORTED;
   const dim3 grid((v.width + kTileW - 1) / kTileW, (v.height + kTileH - 1) / kTileH);
-  if (grid_wide(g))
+  if (g.wide)
     k_grid_layer_grad<true><<<grid, kThreads, 0, s>>>(u, v, g, out);
   else
     k_grid_layer_grad<false><<<grid, kThreads, 0, s>>>(u, v, g, out);

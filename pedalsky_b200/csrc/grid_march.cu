@@ -58,7 +58,7 @@ __device__ __forceinline__ void grid_scatter(const GridDev& g, const Cell<WIDE>&
   const float wy[2] = {1.0f - c.wy, c.wy};
 #pragma unroll
   for (int dy = 0; dy < 2; ++dy)
-    if (wy[dy] != 0.0f)
+    if (wy[dy] != 0.0f && (!WIDE || (dy ? c.hi : c.lo)))
       atomicAdd(g.grads + (c.i + (decltype(c.i))(dy ? g.plane : 0)),
                 make_float4(wy[dy] * q.x, wy[dy] * q.y, wy[dy] * q.z, wy[dy] * q.w));
 }
@@ -432,23 +432,23 @@ __global__ void __launch_bounds__(kThreads, MINB) k_grid_march(const __grid_cons
 
 // One warp per (yi, zi) row of quads, so no index is divided per quad.  Sets
 // *nonfinite when a value is an infinity or NaN.
-__global__ void __launch_bounds__(256) k_grid_quads(const float* __restrict__ v, float4* __restrict__ q,
-                                                    uint32_t nx, uint32_t ny, uint32_t nz,
+__global__ void __launch_bounds__(256) k_grid_quads(const __grid_constant__ GridDev g, float4* __restrict__ q,
                                                     uint32_t* __restrict__ nonfinite) {
-  const uint32_t lane = threadIdx.x & 31u, sz = nz + 3u, sx = nx + 3u;
-  const uint64_t rows = (uint64_t)(ny + 4u) * sz, warps = (uint64_t)gridDim.x * (blockDim.x >> 5);
+  const uint32_t lane = threadIdx.x & 31u, pad = g.pad, sx = g.row, sz = (uint32_t)(g.plane / sx);
+  const uint64_t rows = (uint64_t)(g.ny + 2u * g.pad_y) * sz, warps = (uint64_t)gridDim.x * (blockDim.x >> 5);
   bool bad = false;
   for (uint64_t row = (uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); row < rows; row += warps) {
     const uint32_t yi = (uint32_t)(row / sz), zi = (uint32_t)(row - (uint64_t)yi * sz);
-    const bool in = yi >= 2u && yi - 2u < ny;
-    const bool lo = in && zi >= 2u && zi - 2u < nz, hi = in && zi >= 1u && zi - 1u < nz;  // z = zi - 2 and zi - 1
-    const float* const a = v + ((size_t)(in ? yi - 2u : 0u) * nz + (lo ? zi - 2u : 0u)) * nx;
-    const float* const b = v + ((size_t)(in ? yi - 2u : 0u) * nz + (hi ? zi - 1u : 0u)) * nx;
+    const uint32_t y = yi - g.pad_y, z = zi - pad, z1 = z + 1u;  // outside: at or above the count (mod 2^32)
+    const bool in = y < g.ny, lo = in && z < g.nz, hi = in && z1 < g.nz;
+    const float* const a = g.values + ((size_t)(in ? y : 0u) * g.nz + (lo ? z : 0u)) * g.nx;
+    const float* const b = g.values + ((size_t)(in ? y : 0u) * g.nz + (hi ? z1 : 0u)) * g.nx;
     float4* const out = q + (size_t)row * sx;
     for (uint32_t xi = lane; xi < sx; xi += 32u) {
-      const bool l = xi >= 2u && xi - 2u < nx, r = xi >= 1u && xi - 1u < nx;  // x = xi - 2 and xi - 1
-      const float4 t = make_float4(lo && l ? __ldg(a + xi - 2u) : 0.0f, hi && l ? __ldg(b + xi - 2u) : 0.0f,
-                                   lo && r ? __ldg(a + xi - 1u) : 0.0f, hi && r ? __ldg(b + xi - 1u) : 0.0f);
+      const uint32_t x = xi - pad, x1 = x + 1u;
+      const bool l = x < g.nx, r = x1 < g.nx;
+      const float4 t = make_float4(lo && l ? __ldg(a + x) : 0.0f, hi && l ? __ldg(b + x) : 0.0f,
+                                   lo && r ? __ldg(a + x1) : 0.0f, hi && r ? __ldg(b + x1) : 0.0f);
       bad = bad || !isfinite(t.w);  // every cell is some quad's upper right corner
       out[xi] = t;
     }
@@ -457,30 +457,29 @@ __global__ void __launch_bounds__(256) k_grid_quads(const float* __restrict__ v,
 }
 
 // grad += the four quad entries of each cell, one warp per (y, z) row.
-__global__ void __launch_bounds__(256) k_grid_fold(const float4* __restrict__ gq, float* __restrict__ grad,
-                                                   uint32_t nx, uint32_t ny, uint32_t nz) {
-  const uint32_t lane = threadIdx.x & 31u, warps = gridDim.x * (blockDim.x >> 5), rows = ny * nz, sx = nx + 3u;
+__global__ void __launch_bounds__(256) k_grid_fold(const __grid_constant__ GridDev g) {
+  const uint32_t lane = threadIdx.x & 31u, warps = gridDim.x * (blockDim.x >> 5), rows = g.ny * g.nz;
   for (uint32_t r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); r < rows; r += warps) {
-    const uint32_t y = r / nz, z = r - y * nz;
-    const float4* const up = gq + ((size_t)(y + 2u) * (nz + 3u) + z + 2u) * sx;  // quads whose lower z is z
-    const float4* const dn = up - sx;
-    float* const out = grad + (size_t)r * nx;
-    for (uint32_t x = lane; x < nx; x += 32u)
-      out[x] += (__ldg(up + x + 2u).x + __ldg(up + x + 1u).z) + (__ldg(dn + x + 2u).y + __ldg(dn + x + 1u).w);
+    const uint32_t y = r / g.nz, z = r - y * g.nz;
+    // quads whose lower z is z, from the one whose upper x is 0
+    const float4* const up = g.grads + (size_t)(y + g.pad_y) * g.plane + (size_t)(z + g.pad) * g.row + (g.pad - 1u);
+    const float4* const dn = up - g.row;
+    float* const out = g.grad + (size_t)r * g.nx;
+    for (uint32_t x = lane; x < g.nx; x += 32u)
+      out[x] += (__ldg(up + x + 1u).x + __ldg(up + x).z) + (__ldg(dn + x + 1u).y + __ldg(dn + x).w);
   }
 }
 
 }  // namespace
 
-int launch_grid_quads(const float* values, float4* quads, uint32_t* nonfinite, uint32_t nx, uint32_t ny,
-                      uint32_t nz, cudaStream_t s) {
+int launch_grid_quads(const GridDev& g, float4* quads, uint32_t* nonfinite, cudaStream_t s) {
   if (cudaMemsetAsync(nonfinite, 0, sizeof(uint32_t), s) != cudaSuccess) return PSC_ERR_CUDA;
-  k_grid_quads<<<148u * 8u, 256, 0, s>>>(values, quads, nx, ny, nz, nonfinite);
+  k_grid_quads<<<148u * 8u, 256, 0, s>>>(g, quads, nonfinite);
   return cudaGetLastError() == cudaSuccess ? PSC_OK : PSC_ERR_CUDA;
 }
 
-int launch_grid_fold(const float4* grads, float* grad, uint32_t nx, uint32_t ny, uint32_t nz, cudaStream_t s) {
-  k_grid_fold<<<148u * 8u, 256, 0, s>>>(grads, grad, nx, ny, nz);
+int launch_grid_fold(const GridDev& g, cudaStream_t s) {
+  k_grid_fold<<<148u * 8u, 256, 0, s>>>(g);
   return cudaGetLastError() == cudaSuccess ? PSC_OK : PSC_ERR_CUDA;
 }
 
@@ -489,7 +488,7 @@ int launch_grid_march(const MarchUniforms& u, const ViewDev& v, const GridDev& g
   if (!g.quads || (adjoint && !g.grads)) return PSC_ERR_INVALID_ARGUMENT;
   if (u.octaves == 0 || u.octaves > (uint32_t)kMaxOct) return PSC_ERR_UNSUPPORTED;
   const dim3 grid((v.width + kTileW - 1) / kTileW, (v.height + kTileH - 1) / kTileH);
-  const bool wide = grid_wide(g);
+  const bool wide = g.wide;
   if (adjoint && wide)
     k_grid_march<true, kAdjointCtas, true><<<grid, kThreads, 0, s>>>(u, v, g);
   else if (adjoint)

@@ -2497,9 +2497,7 @@ int prepare_grid(psc_ctx* c, const PscDensityGrid* g, const PscView* v, bool adj
   gd.fnx = not_above(g->nx);
   gd.fny = not_above(g->ny);
   gd.fnz = not_above(g->nz);
-  gd.row = g->nx + 3u;
-  gd.plane = (uint64_t)(g->nz + 3u) * gd.row;
-  gd.origin = (uint32_t)((gd.plane + gd.row + 1u) * 0x4B3FFFFEull);  // 0x4B400000 - 2 per axis
+  psc::set_grid_layout(gd);
   gd.min_x = g->min_x_m;
   gd.min_z = g->min_z_m;
   gd.base = L.base_m;
@@ -2604,7 +2602,7 @@ int grid_call_done(psc_ctx* c, cudaStream_t s) {
 // The grid values as (x, z) corner quads (GridDev::quads) on `s`, and for the
 // adjoint a zeroed gradient of the same form (GridDev::grads).
 int stage_grid_layout(psc_ctx* c, psc::GridDev& gd, bool adjoint, cudaStream_t s) {
-  const size_t nq = (size_t)gd.plane * (gd.ny + 4u);
+  const size_t nq = (size_t)gd.entries();
   RelaxedCapture relaxed;
   float4 *quads = nullptr, *grads = nullptr;
   uint32_t* nonfinite = nullptr;  // behind the quads
@@ -2632,7 +2630,7 @@ int stage_grid_layout(psc_ctx* c, psc::GridDev& gd, bool adjoint, cudaStream_t s
       grads = c->d_grid_grads;
     }
   }
-  if (psc::launch_grid_quads(gd.values, quads, nonfinite, gd.nx, gd.ny, gd.nz, s))
+  if (psc::launch_grid_quads(gd, quads, nonfinite, s))
     return fail(PSC_ERR_CUDA, "grid quad launch failed: %s", cudaGetErrorString(cudaGetLastError()));
   gd.quads = quads;
   gd.nonfinite = nonfinite;
@@ -2681,7 +2679,7 @@ int psc_adjoint(psc_ctx* c, const PscDensityGrid* g, const PscView* v, const flo
   if (rc) return rc;
   rc = psc::launch_grid_march(u, vd, gd, true, s);
   if (rc) return fail(rc, "adjoint launch failed: %s", cudaGetErrorString(cudaGetLastError()));
-  rc = psc::launch_grid_fold(gd.grads, grad_values, gd.nx, gd.ny, gd.nz, s);
+  rc = psc::launch_grid_fold(gd, s);
   if (rc) return fail(rc, "gradient fold launch failed: %s", cudaGetErrorString(cudaGetLastError()));
   ++c->launches;
   return grid_call_done(c, s);

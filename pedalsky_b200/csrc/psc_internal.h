@@ -172,26 +172,49 @@ struct GridDev {
   double* loss;            // adjoint: accumulated loss
   double* grad_scale;      // adjoint: accumulated d loss / d density_scale
   // the values as (x, z) corner quads: entry (yi, zi, xi) holds v[y][z][x],
-  // v[y][z+1][x], v[y][z][x+1], v[y][z+1][x+1] with y = yi - 2, z = zi - 2,
-  // x = xi - 2, zero outside the grid; yi = 0..ny+3, zi = 0..nz+2,
-  // xi = 0..nx+2 (launch_grid_quads).  The adjoint adds its gradient into an
-  // array of the same form (grads), folded into grad afterwards
-  // (launch_grid_fold).
+  // v[y][z+1][x], v[y][z][x+1], v[y][z+1][x+1] with y = yi - pad_y,
+  // z = zi - pad, x = xi - pad, zero outside the grid; yi = 0..ny+2 pad_y-1,
+  // zi = 0..nz+2 pad-2, xi = 0..nx+2 pad-2 (launch_grid_quads).  The adjoint
+  // adds its gradient into an array of the same form (grads), folded into grad
+  // afterwards (launch_grid_fold).
   const float4* quads;
   const uint32_t* nonfinite;  // 1 when the grid holds an infinity or NaN
   float4* grads;
-  uint32_t row;     // entries per row of either array: nx + 3
+  uint32_t wide;        // the kernels of large and thin grids (set_grid_layout)
+  uint32_t pad, pad_y;  // 2, 2; wide: 1, 0
+  uint32_t row;     // entries per row of either array: nx + 2 pad - 1
   uint32_t origin;  // 0x4B3FFFFE x (plane + row + 1) mod 2^32 (grid_cell)
-  uint64_t plane;   // entries per y plane: (nz + 3) (nx + 3)
+  uint64_t plane;   // entries per y plane: (nz + 2 pad - 1) row
+  uint64_t entries() const { return plane * (ny + 2ull * pad_y); }
 };
+// Chooses the arrays' form.  Narrow: two layers of zeros around the grid, so
+// that no fetch tests bounds, counted in 32 bits (floor_bits counts cells
+// exactly up to 2^22).  Wide: only the corners that exist, tested and counted in 64
+// bits: for axes and arrays beyond that, and for large thin grids (over 2^24
+// entries), whose layers of zeros would more than double them: a slab of
+// 32768 x 1 x 32768 cells takes 17 GB an array instead of 86.
+inline void set_grid_layout(GridDev& g) {
+  auto layout = [&g](uint32_t pad, uint32_t pad_y) {
+    g.pad = pad;
+    g.pad_y = pad_y;
+    g.row = g.nx + 2u * pad - 1u;
+    g.plane = (g.nz + 2ull * pad - 1ull) * g.row;
+    return g.entries();
+  };
+  const uint64_t least = layout(1u, 0u), padded = layout(2u, 2u);
+  constexpr uint32_t axis = 1u << 21;
+  g.wide = g.nx >= axis || g.ny >= axis || g.nz >= axis || padded >= (1ull << 31) ||
+           (padded > (1ull << 24) && padded > 2u * least);
+  if (g.wide) layout(1u, 0u);
+  g.origin = (uint32_t)((g.plane + g.row + 1u) * 0x4B3FFFFEull);  // 0x4B400000 - 2 per axis
+}
 int launch_grid_march(const MarchUniforms& u, const ViewDev& v, const GridDev& g, bool adjoint,
                       cudaStream_t stream);
-// GridDev::quads from the ny x nz x nx values; *nonfinite = 1 when a value is
+// `quads` as GridDev::quads from g's values; *nonfinite = 1 when a value is
 // an infinity or NaN, else 0
-// grad += each cell's four entries of grads
-int launch_grid_quads(const float* values, float4* quads, uint32_t* nonfinite, uint32_t nx, uint32_t ny,
-                      uint32_t nz, cudaStream_t stream);
-int launch_grid_fold(const float4* grads, float* grad, uint32_t nx, uint32_t ny, uint32_t nz, cudaStream_t stream);
+// g.grad += each cell's four entries of g.grads
+int launch_grid_quads(const GridDev& g, float4* quads, uint32_t* nonfinite, cudaStream_t stream);
+int launch_grid_fold(const GridDev& g, cudaStream_t stream);
 // d loss / d (base_m, top_m) of layer 0 in the grid form, added to out[0..1]
 // (grid_layer_grad.cu); g.bg / g.target / g.inv_n as for the adjoint.
 int launch_grid_layer_grad(const MarchUniforms& u, const ViewDev& v, const GridDev& g, double* out,
