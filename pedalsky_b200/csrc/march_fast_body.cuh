@@ -210,7 +210,7 @@ __device__ __forceinline__ float2 base_tap(const MarchUniforms& u, float ax, flo
     } else {
       const float k = u.base_texel_scale;
       if constexpr (ST == PSC_STORAGE_U8)
-        b = trilinear_quad_u8<128>(u.base_quad, fmaf(ax, k, -0.5f), fmaf(ay, k, -0.5f), fmaf(az, k, -0.5f));
+        b = trilinear_quad_u8<128>(u.base_quad8, fmaf(ax, k, -0.5f), fmaf(ay, k, -0.5f), fmaf(az, k, -0.5f));
       else
         b = trilinear_texel<ST, 128>(u.noise_base, fmaf(ax, k, -0.5f), fmaf(ay, k, -0.5f),
                                      fmaf(az, k, -0.5f), u.noise_scale);

@@ -68,9 +68,13 @@ struct psc_ctx {
   // F16 storage, FAST schedule: channel-folded volumes (k_fold_* in
   // noise_bake.cu), one texel per entry and 2x2 quads per entry
   uint32_t* d_base_fold = nullptr;   // 128^3 half2 (R, 5G+2B+A)
-  uint4* d_base_quad = nullptr;      // 128^3 x 4 half2 (F16) or RGBA8 texels (U8)
+  uint4* d_base_quad = nullptr;      // 128^3 x 4 half2
   uint16_t* d_detail_fold = nullptr; // 32^3 half (5R+2G+B)
-  uint2* d_detail_quad = nullptr;    // 32^3 x 4 half (F16) or RGBA8 texels (U8, 16 bytes per entry)
+  uint2* d_detail_quad = nullptr;    // 32^3 x 4 half
+  // U8 storage: the RGBA8 texels as quads.  Buffers of their own: a captured
+  // render of one storage form outlives a change to the other
+  uint4* d_base_quad8 = nullptr;     // 128^3 x 4 texels
+  uint4* d_detail_quad8 = nullptr;   // 32^3 x 4 texels
   uint4* d_curl_quad = nullptr;      // 128^2 x 4 half2 (R, G), FAST schedule
 
   // texture-unit path: RGBA8 volumes for U8 storage, the folded volumes for

@@ -486,7 +486,8 @@ void build_uniforms_for(const psc_ctx* c, const PscCloudParamsGpu& p, const PscC
   u.curl_quad = c->d_curl_quad;
   u.base_quad = c->d_base_quad;
   u.detail_quad = c->d_detail_quad;
-  u.detail_quad8 = reinterpret_cast<const uint4*>(c->d_detail_quad);
+  u.base_quad8 = c->d_base_quad8;
+  u.detail_quad8 = c->d_detail_quad8;
   // texture-unit sampling of the transmittance LUT belongs to the filtered
   // forms; EXACT keeps FP32 weights everywhere
   u.tex_trans = c->opts.filter != PSC_FILTER_EXACT ? c->tex_lut[PSC_LUT_TRANSMITTANCE] : 0;
@@ -513,17 +514,18 @@ int build_storage(psc_ctx* c) {
     if (!c->d_curl_quad) PSC_CUDA(cudaMalloc(&c->d_curl_quad, 128u * 128u * 16u), "cudaMalloc curl quads");
     if (psc::launch_curl_quads(c->d_curl, c->d_curl_quad, 0)) return fail(PSC_ERR_CUDA, "curl quad launch failed");
   }
-  if (st == PSC_STORAGE_F16 || st == PSC_STORAGE_U8) {  // both keep their quads in these buffers
-    if (!c->d_base_quad) PSC_CUDA(cudaMalloc(&c->d_base_quad, 128u * 128u * 128u * 16u), "cudaMalloc base quads");
-    if (!c->d_detail_quad) PSC_CUDA(cudaMalloc(&c->d_detail_quad, 32u * 32u * 32u * 16u), "cudaMalloc detail quads");
+  if (st == PSC_STORAGE_U8) {
+    if (!c->d_base_quad8) PSC_CUDA(cudaMalloc(&c->d_base_quad8, 128u * 128u * 128u * 16u), "cudaMalloc base quads");
+    if (!c->d_detail_quad8) PSC_CUDA(cudaMalloc(&c->d_detail_quad8, 32u * 32u * 32u * 16u), "cudaMalloc detail quads");
+    if (psc::launch_quads_u8(c->d_base_u8, c->d_base_quad8, 128u, 0) ||
+        psc::launch_quads_u8(c->d_detail_u8, c->d_detail_quad8, 32u, 0))
+      return fail(PSC_ERR_CUDA, "quad layout launch failed");
   }
-  if (st == PSC_STORAGE_U8 &&
-      (psc::launch_quads_u8(c->d_base_u8, c->d_base_quad, 128u, 0) ||
-       psc::launch_quads_u8(c->d_detail_u8, reinterpret_cast<uint4*>(c->d_detail_quad), 32u, 0)))
-    return fail(PSC_ERR_CUDA, "quad layout launch failed");
   if (st == PSC_STORAGE_F16) {  // the FAST schedule reads the channel-folded forms
     if (!c->d_base_fold) PSC_CUDA(cudaMalloc(&c->d_base_fold, 128u * 128u * 128u * 4u), "cudaMalloc base fold");
+    if (!c->d_base_quad) PSC_CUDA(cudaMalloc(&c->d_base_quad, 128u * 128u * 128u * 16u), "cudaMalloc base quads");
     if (!c->d_detail_fold) PSC_CUDA(cudaMalloc(&c->d_detail_fold, 32u * 32u * 32u * 2u), "cudaMalloc detail fold");
+    if (!c->d_detail_quad) PSC_CUDA(cudaMalloc(&c->d_detail_quad, 32u * 32u * 32u * 8u), "cudaMalloc detail quads");
     if (psc::launch_fold_storage(c->d_base_u8, c->d_detail_u8, c->d_base_fold, c->d_base_quad, c->d_detail_fold,
                                  c->d_detail_quad, 0))
       return fail(PSC_ERR_CUDA, "channel fold launch failed");
@@ -1562,6 +1564,8 @@ int psc_destroy(psc_ctx* c) {
   dfree(c->d_base_quad);
   dfree(c->d_detail_fold);
   dfree(c->d_detail_quad);
+  dfree(c->d_base_quad8);
+  dfree(c->d_detail_quad8);
   dfree(c->d_curl_quad);
   dfree(c->d_curl);
   dfree(c->d_rt_l);

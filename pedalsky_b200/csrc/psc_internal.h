@@ -136,9 +136,10 @@ struct alignas(16) MarchUniforms {
   // the noise volumes as 2x2 (x, y) quads per entry: F16 storage (FAST
   // schedule) the channel-folded (R, fbm) and (detail fbm)
   // (noise_bake.cu:k_fold_*), U8 storage the RGBA8 texels (k_quads_u8)
-  const uint4* base_quad;
-  const uint2* detail_quad;    // F16
-  const uint4* detail_quad8;   // U8
+  const uint4* base_quad;      // F16
+  const uint2* detail_quad;
+  const uint4* base_quad8;     // U8
+  const uint4* detail_quad8;
   const uint4* curl_quad;      // FAST schedule: curl tile as 2x2 (R, G) half quads
   // transmittance / sky-view LUTs through the texture unit; 0 = plain loads
   cudaTextureObject_t tex_trans, tex_sky;
