@@ -490,7 +490,7 @@ typedef struct PscFetchCounts {
   uint64_t type_loads;          /* cloud-type grid loads                   */
   uint64_t detail_taps;         /* trilinear detail taps                   */
   uint64_t dense_samples;       /* samples with density > 1e-3             */
-  uint64_t light_taps;          /* light-march base taps                   */
+  uint64_t light_taps;          /* light-march base taps fetched           */
   uint64_t transmittance_taps;  /* transmittance-LUT taps (sunlit samples) */
   uint64_t skyview_taps;        /* sky-view LUT taps                       */
   uint64_t ap_taps;             /* aerial-perspective taps                 */

@@ -110,6 +110,8 @@ enum {
   ORACLE_CNT_STEPS,        /* primary steps executed                      */
   ORACLE_CNT_DENSE,        /* dense (density > 1e-3) primary steps        */
   ORACLE_CNT_PIXELS,
+  ORACLE_CNT_LIGHT_LIVE,   /* LIGHT taps whose profile exceeds 1 - eff: the
+                              others' density is 0 whatever the noise       */
   ORACLE_CNT__COUNT
 };
 

@@ -369,6 +369,7 @@ struct March {
                            R(0), R(1));
     const R base_cloud = remap<R>(base[0], -(R(1) - lf), R(1), R(0), R(1));
     const R profile = ndf(h, type, L.anvil_bias);
+    if (light && profile > R(1) - eff_cov) count(ORACLE_CNT_LIGHT_LIVE);
     R cloud = base_cloud * profile;
     cloud = remap<R>(cloud, R(1) - eff_cov, R(1), R(0), R(1));
     return cloud * eff_cov;

@@ -21,7 +21,7 @@ LIB_PATH = HERE / "liboracle.so"
 FP32, FP64 = 32, 64
 FILTER_EXACT, FILTER_Q8 = 0, 1
 COUNTERS = ("weather", "type", "base", "curl", "detail", "light", "trans", "sky", "wind", "ap",
-            "blue", "depth", "steps", "dense", "pixels")
+            "blue", "depth", "steps", "dense", "pixels", "light_live")
 
 
 class OracleScene(C.Structure):

@@ -321,10 +321,12 @@ __device__ __forceinline__ float ndf_eval(const NdfCoef& k, float h) {
   return ssr_b(k.inv_a, 0.0f, h) * ssr_b(k.inv_w1, k.b1, h);
 }
 
-template <int ST, int FILT>
+// `taps` (the instrumented build's, else none): counts the tap where it is
+// fetched.
+template <int ST, int FILT, class... Taps>
 __device__ __forceinline__ float density_light(const MarchUniforms& u, const LayerConst& L, float qx,
                                                float qy, float qz, float alt, float eff,
-                                               uint32_t type) {
+                                               uint32_t type, Taps... taps) {
   const float h = (alt - L.base_m) * L.inv_thickness;
   if (h < 0.0f || h > 1.0f) return 0.0f;
   // the base shape is at most 1: where the profile does not reach 1 - eff the
@@ -334,6 +336,7 @@ __device__ __forceinline__ float density_light(const MarchUniforms& u, const Lay
   if (!(nd * 1.000001f > 1.0f - eff)) return 0.0f;
   const float ax = fmaf(-L.skew_kx, h, qx - L.wind_off_x);
   const float az = fmaf(-L.skew_kz, h, qz - L.wind_off_z);
+  ((++*taps), ...);
   const float2 b = base_tap<ST, FILT, true>(u, ax, qy, az);
   return clamp01(shape_from<ST>(b, L.lf_c, nd, 1.0f - eff)) * L.density_scale;
 }
@@ -346,10 +349,10 @@ __device__ __forceinline__ float alt_from(const MarchUniforms& u, float qx, floa
   return h0 + __fdividef(num, r0 + len);
 }
 
-template <int ST, int FILT>
+template <int ST, int FILT, class... Taps>
 __device__ __noinline__ float light_cone(const MarchUniforms& u, const LayerConst& L, float px,
                                          float py, float pz, float alt, float eff, uint32_t type,
-                                         float r0, float cv, float dist) {
+                                         float r0, float cv, float dist, Taps... taps) {
   const float K[6][3] = {{0.38051305f, 0.92453449f, -0.02111345f},
                          {-0.50625799f, -0.03590792f, -0.86163418f},
                          {-0.32509218f, -0.94557439f, 0.01428793f},
@@ -367,14 +370,14 @@ __device__ __noinline__ float light_cone(const MarchUniforms& u, const LayerCons
     const float qy = fmaf(sy, t, py) + K[i][1] * sc;
     const float qz = fmaf(sz, t, pz) + K[i][2] * sc;
     od += density_light<ST, FILT>(u, L, qx, qy, qz, alt_from(u, qx, qy, qz, r0, cv, alt, t), eff,
-                                  type) * step;
+                                  type, taps...) * step;
   }
   const float tf = dist * 3.0f;
   const float qx = fmaf(sx, tf, px) + K[5][0] * (step * 3.0f);
   const float qy = fmaf(sy, tf, py) + K[5][1] * (step * 3.0f);
   const float qz = fmaf(sz, tf, pz) + K[5][2] * (step * 3.0f);
   od += density_light<ST, FILT>(u, L, qx, qy, qz, alt_from(u, qx, qy, qz, r0, cv, alt, tf), eff,
-                                type) * step * 3.0f;
+                                type, taps...) * step * 3.0f;
   return od;
 }
 
@@ -542,10 +545,10 @@ __device__ __forceinline__ float light_march_tex(const MarchUniforms& u, const L
   return od;
 }
 
-// Optical depth toward the sun (cloud_march.wgsl:543-578).  `taps`, when
-// given, is lowered to the number of taps fetched where the lean form's
-// light march stops early.
-template <int ST, int FILT, int FORM = kFormFull, int LB = 0>
+// Optical depth toward the sun (cloud_march.wgsl:543-578).  TALLY: `taps`
+// becomes the number of taps fetched where that is not all of them (the lean
+// form's light march stops early, density_light leaves taps out).
+template <int ST, int FILT, int FORM = kFormFull, int LB = 0, bool TALLY = false>
 __device__ __forceinline__ float light_od(const MarchUniforms& u, const LayerConst& L, float px,
                                           float py, float pz, float alt, float eff, uint32_t type,
                                           float ux, float uy, float uz, uint32_t* taps = nullptr) {
@@ -554,7 +557,16 @@ __device__ __forceinline__ float light_od(const MarchUniforms& u, const LayerCon
   const float r0 = u.planet_r + alt;
   const float cv = fmaf(ux, u.sun[0], fmaf(uy, u.sun[1], uz * u.sun[2]));
   const float dist = fmaxf((L.top_m - alt) * u.inv_cos_sun, 1.0f);
-  if (FULL && u.cone) return light_cone<ST, FILT>(u, L, px, py, pz, alt, eff, type, r0, cv, dist);
+  if constexpr (FULL) {
+    if (u.cone) {
+      if constexpr (TALLY) {
+        *taps = 0u;
+        return light_cone<ST, FILT>(u, L, px, py, pz, alt, eff, type, r0, cv, dist, taps);
+      } else {
+        return light_cone<ST, FILT>(u, L, px, py, pz, alt, eff, type, r0, cv, dist);
+      }
+    }
+  }
   const float step = __fdividef(dist, (float)u.light_steps);
   if constexpr (FILT != PSC_FILTER_EXACT) {
     const float k = u.inv_base_scale;
@@ -596,12 +608,14 @@ __device__ __forceinline__ float light_od(const MarchUniforms& u, const LayerCon
     return light_march_tex<ST, NdfGeneral, false, false, FULL, LB>(u, L, lr, gen);
   }
   float od = 0.0f, comp = 0.0f;
+  if constexpr (TALLY) *taps = 0u;
   for (uint32_t i = 0; i < u.light_steps; ++i) {
     const float t = ((float)i + 0.5f) * step;
     const float qx = fmaf(u.sun[0], t, px), qy = fmaf(u.sun[1], t, py), qz = fmaf(u.sun[2], t, pz);
-    const float term =
-        density_light<ST, FILT>(u, L, qx, qy, qz, alt_from(u, qx, qy, qz, r0, cv, alt, t), eff, type) *
-        step;
+    const float a = alt_from(u, qx, qy, qz, r0, cv, alt, t);
+    float term;
+    if constexpr (TALLY) term = density_light<ST, FILT>(u, L, qx, qy, qz, a, eff, type, taps) * step;
+    else term = density_light<ST, FILT>(u, L, qx, qy, qz, a, eff, type) * step;
     if (FULL && u.kahan) {
       const float y = term - comp;
       const float tt = od + y;
@@ -926,7 +940,7 @@ __device__ __forceinline__ void march_pixel_fast(const MarchUniforms& u, const V
               tc[kTallyTrans] += trans_fetched ? 1u : 0u;
             }
             uint32_t light_taps_done = (FULL && u.cone) ? 6u : u.light_steps;
-            const float od = light_od<ST, FILT, FORM, LB>(u, L, px3, py3, pz3, alt, eff, type, ux, uy, uz,
+            const float od = light_od<ST, FILT, FORM, LB, TALLY>(u, L, px3, py3, pz3, alt, eff, type, ux, uy, uz,
                                                           TALLY ? &light_taps_done : nullptr);
             if constexpr (TALLY) tc[kTallyLight] += light_taps_done;
             const float st_r = L.sigma_t[0], st_g = L.sigma_t[1], st_b = L.sigma_t[2];
