@@ -1,7 +1,8 @@
 // Single-view FAST march kernel: one thread per ray, CTA tile 16x8 pixels,
 // warps as 8x4 pixel tiles, 8 CTAs per SM for the lean form (64 registers:
 // more resident warps hide more fetch latency than the few spilled values
-// cost) and 7 for the others (72 registers: their extra paths spill more).
+// cost), 7 for the others (72 registers: their extra paths spill more) and 5 for
+// launches of few CTAs of the Cumulonimbus form.
 // One 4K frame under a Cumulonimbus layer, 256 + 8 steps: 9.21 ms in the full
 // form, 8.83 in the Cumulonimbus form (8.98 at 8 CTAs per SM, 9.14 at 6), 8.58
 // with its profile's plateau tested first.  The per-ray
@@ -20,10 +21,14 @@ constexpr int kThreads = 128;
 
 // The form a march over this uniform block takes: lean without Cumulonimbus
 // layers, a cloud-type grid, Kahan sums, cone sampling and lightning; with
-// Cumulonimbus as the only one of them its own, in its form for few CTAs up to
-// one per SM (110 CTAs are slower with the plateau, 255 even, 510 faster); full
-// otherwise.
-constexpr uint32_t kFewCtas = 148;
+// Cumulonimbus as the only one of them its own; full otherwise.  Launches whose
+// CTAs are all resident at 7 per SM gain nothing from that many and take the
+// Cumulonimbus form compiled for 5 (92 registers, no spills, no plateau branch):
+// there one ray's chain of latencies is the time.  256 + 8 steps, form of 7 /
+// of 5 per SM: 96x54 560 / 501 us, 240x135 (255 CTAs) 505 / 457, 400x225 (725)
+// 520 / 481, 480x270 (1020) 549 / 519; beyond, 560x315 (1400) 576 / 535, 640x360
+// (1800) 602 / 654.
+constexpr uint32_t kFewCtas = 148 * 7;
 int kernel_form(const MarchUniforms& u, const dim3& grid) {
   if (!needs_full_paths(&u, 1)) return kFormLean;
   if (u.type_grid || u.kahan || u.cone || u.lightning_radius > 0.0f) return kFormFull;
@@ -33,8 +38,8 @@ int kernel_form(const MarchUniforms& u, const dim3& grid) {
 // Shared memory per CTA: the entry/exit distances of each of the view's
 // layers and kAuxWords more words, per thread (dynamic, sized at launch).
 template <int ST, int FILT, int FORM, int LB>
-__global__ void __launch_bounds__(kThreads, FORM == kFormLean ? 8 : 7) k_march_fast(const __grid_constant__ MarchUniforms u,
-                                                            const __grid_constant__ ViewDev v) {
+__global__ void __launch_bounds__(kThreads, FORM == kFormLean ? 8 : FORM == kFormCumulonimbusFew ? 5 : 7)
+    k_march_fast(const __grid_constant__ MarchUniforms u, const __grid_constant__ ViewDev v) {
   extern __shared__ float s_dyn[];
   const uint32_t nl = u.layer_count;
   float* const s_t0 = s_dyn;
