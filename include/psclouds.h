@@ -628,8 +628,9 @@ typedef struct PscDensityGrid {
  * Needs the frame, blue noise and the transmittance and sky-view LUTs.
  *
  * Grid calls (this one, psc_adjoint, psc_layer_gradient) of one context may
- * be queued on any streams: they share scratch that grows to the largest grid
- * and run one after the other.  A call on a capturing stream takes scratch of
+ * be queued on any streams.  They stage the grid into scratch that the context
+ * keeps, up to eight times for calls in flight on as many streams (once for
+ * grids of over 2^23 cells, whose calls run one after the other).  A call on a capturing stream takes scratch of
  * its own (16 bytes per cell, 32 for the adjoint), which its graph keeps until
  * the graph and its executables are destroyed, so a graph may be replayed
  * beside other grid calls and other graphs; two launches of the same captured

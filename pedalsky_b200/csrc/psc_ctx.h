@@ -119,14 +119,21 @@ struct psc_ctx {
   float4* d_bsky = nullptr;             // per-view sky-view LUTs
   std::vector<cudaTextureObject_t> batch_sky_tex;  // per-view sky-view LUTs through the texture unit
   float4* d_bap = nullptr;              // per-view aerial-perspective LUTs
-  // voxel-grid form: the grid values as corner quads and the adjoint's
+  // voxel-grid form: a call's grid values as corner quads and the adjoint's
   // gradient in the same form (GridDev::quads / grads), each grown to the
-  // largest grid seen; GridDev::nonfinite lies behind the quads
-  float4* d_grid_quads = nullptr;
-  float4* d_grid_grads = nullptr;
-  cudaEvent_t grid_done = nullptr;  // the last grid call's end: the next one, on whatever stream, waits for it
+  // largest grid seen; GridDev::nonfinite lies behind the quads.  One slot for
+  // each stream that has calls in flight (grid_slot)
+  struct GridSlot {
+    float4* quads = nullptr;
+    float4* grads = nullptr;
+    size_t quads_cap = 0, grads_cap = 0;  // entries
+    cudaEvent_t done = nullptr;           // the slot's last call's end: the next one waits for it
+    cudaStream_t stream = nullptr;        // that call's
+  };
+  static constexpr uint32_t kGridSlots = 8;
+  GridSlot grid_slots[kGridSlots];
+  uint32_t grid_turn = 0;
   psc::host::GraphScratch* graph_scratch = nullptr;  // of captured grid calls
-  size_t grid_quads_cap = 0, grid_grads_cap = 0;  // entries
   uint32_t* d_btiles = nullptr;
   uint32_t* d_bcounter = nullptr;
   psc::MarchUniforms* h_bu = nullptr;   // pinned staging

@@ -1572,10 +1572,12 @@ int psc_destroy(psc_ctx* c) {
   dfree(c->d_rt_t);
   dfree(c->d_rt_depth);
   dfree(c->d_check);
-  dfree(c->d_grid_quads);
-  dfree(c->d_grid_grads);
-  if (c->grid_done) cudaEventDestroy(c->grid_done);
-  c->grid_done = nullptr;
+  for (auto& slot : c->grid_slots) {
+    dfree(slot.quads);
+    dfree(slot.grads);
+    if (slot.done) cudaEventDestroy(slot.done);
+    slot.done = nullptr;
+  }
   while (GraphScratch* g = c->graph_scratch) {  // a graph still there must not be launched any more
     c->graph_scratch = g->next;
     cudaFree(g->p);
@@ -2592,24 +2594,45 @@ int graph_scratch(psc_ctx* c, size_t bytes, cudaStream_t s, void** out) {
   return PSC_OK;
 }
 
-// The grid calls of a context share its quads: each marks its end on its
-// stream, and the next one waits for that.  A captured call has its graph's
-// own and needs neither.
-int grid_call_done(psc_ctx* c, cudaStream_t s) {
-  if (capturing(s)) return PSC_OK;
-  if (!c->grid_done)
-    PSC_CUDA(cudaEventCreateWithFlags(&c->grid_done, cudaEventDisableTiming), "grid event");
-  PSC_CUDA(cudaEventRecord(c->grid_done, s), "grid event record");
-  return PSC_OK;
+// The slot of a call of `n` entries on `s`: the one of the last call on that
+// stream, else one whose last call has ended, else the next in turn, whose
+// last call it waits for.  A view of a few CTAs leaves most of the device to
+// the calls on other streams (97^2 rays: 220 us a call on one stream, on
+// eight streams 220 us a call in one slot); a call of over 2^23 entries (134
+// MB) fills it and takes the first slot.
+psc_ctx::GridSlot& grid_slot(psc_ctx* c, size_t n, cudaStream_t s) {
+  if (n > (1u << 23)) return c->grid_slots[0];
+  for (auto& slot : c->grid_slots)
+    if (slot.done && slot.stream == s) return slot;
+  psc_ctx::GridSlot* idle = nullptr;
+  for (auto& slot : c->grid_slots)
+    if (!idle && (!slot.done || cudaEventQuery(slot.done) == cudaSuccess)) idle = &slot;
+  cudaGetLastError();  // a call still in flight
+  return idle ? *idle : c->grid_slots[c->grid_turn++ % psc_ctx::kGridSlots];
+}
+
+// Room for `n` entries in the slot, after its last call.
+int reserve_grid_slot(psc_ctx::GridSlot& slot, size_t n, bool adjoint, cudaStream_t s) {
+  if (slot.done) PSC_CUDA(cudaStreamWaitEvent(s, slot.done, 0), "grid event wait");
+  else PSC_CUDA(cudaEventCreateWithFlags(&slot.done, cudaEventDisableTiming), "grid event");
+  if (slot.quads_cap < n) {
+    dfree(slot.quads);
+    slot.quads_cap = 0;
+    PSC_CUDA(cudaMalloc(&slot.quads, (n + 1u) * sizeof(float4)), "cudaMalloc grid quads");  // + the flag
+    slot.quads_cap = n;
+  }
+  return adjoint ? grow(&slot.grads, &slot.grads_cap, n, "cudaMalloc gradient quads") : PSC_OK;
 }
 
 // The grid values as (x, z) corner quads (GridDev::quads) on `s`, and for the
-// adjoint a zeroed gradient of the same form (GridDev::grads).
-int stage_grid_layout(psc_ctx* c, psc::GridDev& gd, bool adjoint, cudaStream_t s) {
+// adjoint a zeroed gradient of the same form (GridDev::grads).  `*used`: the
+// slot they are in, none for a captured call.
+int stage_grid_layout(psc_ctx* c, psc::GridDev& gd, bool adjoint, cudaStream_t s, psc_ctx::GridSlot** used) {
   const size_t nq = (size_t)gd.entries();
   RelaxedCapture relaxed;
   float4 *quads = nullptr, *grads = nullptr;
   uint32_t* nonfinite = nullptr;  // behind the quads
+  *used = nullptr;
   if (capturing(s)) {
     void* p = nullptr;
     const int rc = graph_scratch(c, (nq * (adjoint ? 2u : 1u) + 1u) * sizeof(float4), s, &p);
@@ -2619,20 +2642,19 @@ int stage_grid_layout(psc_ctx* c, psc::GridDev& gd, bool adjoint, cudaStream_t s
     grads = adjoint ? quads + nq + 1u : nullptr;
   } else {
     idle_graph_scratch(c, 0);
-    if (c->grid_done) PSC_CUDA(cudaStreamWaitEvent(s, c->grid_done, 0), "grid event wait");
-    if (c->grid_quads_cap < nq) {
-      dfree(c->d_grid_quads);
-      c->grid_quads_cap = 0;
-      PSC_CUDA(cudaMalloc(&c->d_grid_quads, (nq + 1u) * sizeof(float4)), "cudaMalloc grid quads");
-      c->grid_quads_cap = nq;
+    psc_ctx::GridSlot* slot = &grid_slot(c, nq, s);
+    int rc = reserve_grid_slot(*slot, nq, adjoint, s);
+    if (rc && slot != c->grid_slots) {  // no memory for one more
+      cudaGetLastError();
+      slot = c->grid_slots;
+      rc = reserve_grid_slot(*slot, nq, adjoint, s);
     }
-    quads = c->d_grid_quads;
-    nonfinite = reinterpret_cast<uint32_t*>(quads + c->grid_quads_cap);
-    if (adjoint) {
-      const int rc = grow(&c->d_grid_grads, &c->grid_grads_cap, nq, "cudaMalloc gradient quads");
-      if (rc) return rc;
-      grads = c->d_grid_grads;
-    }
+    if (rc) return rc;
+    quads = slot->quads;
+    nonfinite = reinterpret_cast<uint32_t*>(quads + slot->quads_cap);
+    grads = slot->grads;
+    slot->stream = s;
+    *used = slot;
   }
   if (psc::launch_grid_quads(gd, quads, nonfinite, s))
     return fail(PSC_ERR_CUDA, "grid quad launch failed: %s", cudaGetErrorString(cudaGetLastError()));
@@ -2642,6 +2664,11 @@ int stage_grid_layout(psc_ctx* c, psc::GridDev& gd, bool adjoint, cudaStream_t s
     PSC_CUDA(cudaMemsetAsync(grads, 0, nq * sizeof(float4), s), "gradient quad reset");
     gd.grads = grads;
   }
+  return PSC_OK;
+}
+
+int grid_call_done(psc_ctx::GridSlot* slot, cudaStream_t s) {
+  if (slot) PSC_CUDA(cudaEventRecord(slot->done, s), "grid event record");
   return PSC_OK;
 }
 
@@ -2655,12 +2682,13 @@ int psc_render_grid(psc_ctx* c, const PscDensityGrid* g, const PscView* v, void*
   psc::GridDev gd;
   int rc = prepare_grid(c, g, v, false, u, vd, gd);
   if (rc) return rc;
-  rc = stage_grid_layout(c, gd, false, static_cast<cudaStream_t>(stream));
+  psc_ctx::GridSlot* slot = nullptr;
+  rc = stage_grid_layout(c, gd, false, static_cast<cudaStream_t>(stream), &slot);
   if (rc) return rc;
   rc = psc::launch_grid_march(u, vd, gd, false, static_cast<cudaStream_t>(stream));
   if (rc) return fail(rc, "grid march launch failed: %s", cudaGetErrorString(cudaGetLastError()));
   ++c->launches;
-  return grid_call_done(c, static_cast<cudaStream_t>(stream));
+  return grid_call_done(slot, static_cast<cudaStream_t>(stream));
 }
 
 int psc_adjoint(psc_ctx* c, const PscDensityGrid* g, const PscView* v, const float* background,
@@ -2679,14 +2707,15 @@ int psc_adjoint(psc_ctx* c, const PscDensityGrid* g, const PscView* v, const flo
   gd.loss = loss;
   gd.grad_scale = grad_density_scale;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  rc = stage_grid_layout(c, gd, true, s);
+  psc_ctx::GridSlot* slot = nullptr;
+  rc = stage_grid_layout(c, gd, true, s, &slot);
   if (rc) return rc;
   rc = psc::launch_grid_march(u, vd, gd, true, s);
   if (rc) return fail(rc, "adjoint launch failed: %s", cudaGetErrorString(cudaGetLastError()));
   rc = psc::launch_grid_fold(gd, s);
   if (rc) return fail(rc, "gradient fold launch failed: %s", cudaGetErrorString(cudaGetLastError()));
   ++c->launches;
-  return grid_call_done(c, s);
+  return grid_call_done(slot, s);
 }
 
 int psc_layer_gradient(psc_ctx* c, const PscDensityGrid* g, const PscView* v, const float* background,
@@ -2709,12 +2738,13 @@ int psc_layer_gradient(psc_ctx* c, const PscDensityGrid* g, const PscView* v, co
   u.tex_sky = 0;
   gd.bg = reinterpret_cast<const float4*>(background);
   gd.target = reinterpret_cast<const float4*>(target);
-  rc = stage_grid_layout(c, gd, false, static_cast<cudaStream_t>(stream));
+  psc_ctx::GridSlot* slot = nullptr;
+  rc = stage_grid_layout(c, gd, false, static_cast<cudaStream_t>(stream), &slot);
   if (rc) return rc;
   rc = psc::launch_grid_layer_grad(u, vd, gd, grad_base_top, static_cast<cudaStream_t>(stream));
   if (rc) return fail(rc, "layer-gradient launch failed: %s", cudaGetErrorString(cudaGetLastError()));
   ++c->launches;
-  return grid_call_done(c, static_cast<cudaStream_t>(stream));
+  return grid_call_done(slot, static_cast<cudaStream_t>(stream));
 }
 
 int psc_layer_param_gradient(psc_ctx* c, const PscView* v, uint32_t layer, const float* background,
