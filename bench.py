@@ -407,7 +407,7 @@ def grid_cpu_sample(sc, noise, luts, rows: int):
     return 4 * band * sc.width, time.perf_counter() - t0, threads
 
 
-GRID_METRIC = ("Mrays/s of the adjoint (forward + checkpointed reverse + gradient all-reduce), "
+GRID_METRIC = ("Mrays/s of the adjoint (forward + reverse sweep + gradient all-reduce), "
                "512^2 view of a 256x256x64 voxel grid, 96+6 steps")
 
 

@@ -21,10 +21,11 @@
 // sum of the grid values of the steps before it: the forward march sums them
 // in FP64 and the reverse sweep takes each step's value off again, each held to
 // what makes a step opaque (`cap`) so that no value is lost beside a larger one
-// (2^-53 of 256 such steps is 1e-11 of optical depth).  Neither checkpoints nor
-// a recomputed segment are needed and the L1 has no shared memory to make room for (checkpoints and
-// segment buffers in 25.6 KB of shared memory per CTA: 1886 us, without: 1668
-// us; each KB per CTA more cost about 20 us).  d loss / d density at the
+// (2^-53 of 256 such steps is 1e-11 of optical depth; 1341 -> 1359 us).  Neither
+// checkpoints nor a recomputed segment are needed and the L1 has no shared
+// memory to make room for (checkpoints and segment buffers in 25.6 KB of shared
+// memory per CTA: 1886 us, without: 1668 us; each KB per CTA more cost about 20
+// us).  d loss / d density at the
 // primary sample and d loss / d optical depth toward the sun are scattered
 // into the gradient with vector atomic adds over the trilinear weights of the
 // primary sample and of the six light taps, one 16-byte add per y row (as

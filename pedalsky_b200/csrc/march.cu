@@ -14,13 +14,14 @@
 // same: the phase values of the octaves (per ray and layer), the uniform
 // weather tap, the steps and light taps whose profile value cannot reach the
 // coverage (they add exactly 0 or stay under the density threshold), the first
-// octave's exponentials (those of Beer's law), and general divisions by what
-// is fixed (div_by).  1920x1080, three layers, 128 + 6 steps, 8-bit noise:
-// 32.1 -> 14.0 ms (20.2 G to 10.5 G warp instructions), the transmittance bit
-// for bit and the luminance within 1.2e-7.  It stays bound by instructions, a
-// good part of them fetches of the instructions themselves (the IEEE square
-// roots, divisions and arctangents of a dense sample make a body larger than
-// the instruction cache: 1.3 stalls per issue, 2.4 before).
+// octave's exponentials (those of Beer's law), and general divisions and roots,
+// which are multiply-adds with the IEEE result (div_by, div_near, sqrt_near).
+// 1920x1080, three layers, 128 + 6 steps, 8-bit noise: 32.1 -> 12.8 ms; on that
+// frame the transmittance came out bit for bit and the luminance within 2.4e-7.
+// It stays bound by instructions, a good part of them fetches of the
+// instructions themselves (a dense sample's exponentials, arctangents and
+// lookups make a body larger than the instruction cache: 1.4 stalls per issue,
+// 2.4 before).
 #include <cuda_runtime.h>
 #include <stdint.h>
 
