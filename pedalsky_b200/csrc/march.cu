@@ -307,7 +307,10 @@ int launch_march(const MarchUniforms& u, const ViewDev& v, const PscMarchOptions
     e = launch_plain<PSC_STORAGE_U8, PSC_FILTER_TEXTURE>(u, v, s);
   } else {
     switch (o.storage) {
-      case PSC_STORAGE_U8: e = launch_plain<PSC_STORAGE_U8, PSC_FILTER_EXACT>(u, v, s); break;
+      case PSC_STORAGE_U8:
+        e = u.far_texels ? launch_plain<kStorageU8Far, PSC_FILTER_EXACT>(u, v, s)
+                         : launch_plain<PSC_STORAGE_U8, PSC_FILTER_EXACT>(u, v, s);
+        break;
       case PSC_STORAGE_F32: e = launch_plain<PSC_STORAGE_F32, PSC_FILTER_EXACT>(u, v, s); break;
       case PSC_STORAGE_F16: e = launch_plain<PSC_STORAGE_F16, PSC_FILTER_EXACT>(u, v, s); break;
       case PSC_STORAGE_BF16: e = launch_plain<PSC_STORAGE_BF16, PSC_FILTER_EXACT>(u, v, s); break;

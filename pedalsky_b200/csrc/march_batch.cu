@@ -112,7 +112,7 @@ int launch_batch_nt(int nt, const MarchUniforms* u, const ViewDev* v, const uint
 
 int launch_march_batch(const PscMarchOptions& o, int threads, uint32_t tile_w,
                        const MarchUniforms* u, const ViewDev* v, const uint32_t* tiles,
-                       uint32_t n_tiles, uint32_t* counter, int sms, bool full, cudaStream_t s) {
+                       uint32_t n_tiles, uint32_t* counter, int sms, bool full, bool far, cudaStream_t s) {
   if (o.filter == PSC_FILTER_HYBRID) {
     // the light-march fetch batch is chosen for the F16 hybrid form only
     if (o.storage == PSC_STORAGE_F16 && o.light_batch == 2)
@@ -127,7 +127,8 @@ int launch_march_batch(const PscMarchOptions& o, int threads, uint32_t tile_w,
     if (o.storage == PSC_STORAGE_F16)
       return launch_batch_nt<PSC_STORAGE_F16, PSC_FILTER_EXACT>(threads, u, v, tiles, n_tiles, counter, tile_w, sms, full, s);
     if (o.storage == PSC_STORAGE_U8)
-      return launch_batch_nt<PSC_STORAGE_U8, PSC_FILTER_EXACT>(threads, u, v, tiles, n_tiles, counter, tile_w, sms, full, s);
+      return far ? launch_batch_nt<kStorageU8Far, PSC_FILTER_EXACT>(threads, u, v, tiles, n_tiles, counter, tile_w, sms, full, s)
+                 : launch_batch_nt<PSC_STORAGE_U8, PSC_FILTER_EXACT>(threads, u, v, tiles, n_tiles, counter, tile_w, sms, full, s);
     if (o.storage == PSC_STORAGE_F32)
       return launch_batch_nt<PSC_STORAGE_F32, PSC_FILTER_EXACT>(threads, u, v, tiles, n_tiles, counter, tile_w, sms, full, s);
   } else if (o.filter == PSC_FILTER_TEXTURE) {

@@ -121,7 +121,8 @@ int launch_march_fast_tally(const MarchUniforms& u, const ViewDev& v, const PscM
   else if (o.storage == PSC_STORAGE_U8 && o.filter == PSC_FILTER_HYBRID)
     e = launch_fast_tally<PSC_STORAGE_U8, PSC_FILTER_HYBRID>(u, v, counts, s);
   else if (o.storage == PSC_STORAGE_U8 && o.filter == PSC_FILTER_EXACT)
-    e = launch_fast_tally<PSC_STORAGE_U8, PSC_FILTER_EXACT>(u, v, counts, s);
+    e = u.far_texels ? launch_fast_tally<kStorageU8Far, PSC_FILTER_EXACT>(u, v, counts, s)
+                     : launch_fast_tally<PSC_STORAGE_U8, PSC_FILTER_EXACT>(u, v, counts, s);
   else
     return PSC_ERR_UNSUPPORTED;
   return e == cudaSuccess ? PSC_OK : PSC_ERR_CUDA;
@@ -146,7 +147,10 @@ int launch_march_fast(const MarchUniforms& u, const ViewDev& v, const PscMarchOp
     else return PSC_ERR_UNSUPPORTED;
   } else {
     switch (o.storage) {
-      case PSC_STORAGE_U8: e = launch_fast<PSC_STORAGE_U8, PSC_FILTER_EXACT>(u, v, s); break;
+      case PSC_STORAGE_U8:
+        e = u.far_texels ? launch_fast<kStorageU8Far, PSC_FILTER_EXACT>(u, v, s)
+                         : launch_fast<PSC_STORAGE_U8, PSC_FILTER_EXACT>(u, v, s);
+        break;
       case PSC_STORAGE_F32: e = launch_fast<PSC_STORAGE_F32, PSC_FILTER_EXACT>(u, v, s); break;
       case PSC_STORAGE_F16: e = launch_fast<PSC_STORAGE_F16, PSC_FILTER_EXACT>(u, v, s); break;
       case PSC_STORAGE_BF16: e = launch_fast<PSC_STORAGE_BF16, PSC_FILTER_EXACT>(u, v, s); break;

@@ -209,8 +209,9 @@ __device__ __forceinline__ float2 base_tap(const MarchUniforms& u, float ax, flo
                         az * u.inv_base_scale);
     } else {
       const float k = u.base_texel_scale;
-      if constexpr (ST == PSC_STORAGE_U8)
-        b = trilinear_quad_u8<128>(u.base_quad8, fmaf(ax, k, -0.5f), fmaf(ay, k, -0.5f), fmaf(az, k, -0.5f));
+      if constexpr (ST == PSC_STORAGE_U8 || ST == kStorageU8Far)
+        b = trilinear_quad_u8<128, ST == kStorageU8Far>(u.base_quad8, fmaf(ax, k, -0.5f), fmaf(ay, k, -0.5f),
+                                                        fmaf(az, k, -0.5f));
       else
         b = trilinear_texel<ST, 128>(u.noise_base, fmaf(ax, k, -0.5f), fmaf(ay, k, -0.5f),
                                      fmaf(az, k, -0.5f), u.noise_scale);
@@ -237,8 +238,9 @@ __device__ __forceinline__ float detail_tap(const MarchUniforms& u, float dx, fl
                         dz * u.inv_detail_scale);
     } else {
       const float k = u.detail_texel_scale;
-      if constexpr (ST == PSC_STORAGE_U8)
-        d = trilinear_quad_u8<32>(u.detail_quad8, fmaf(dx, k, -0.5f), fmaf(dy, k, -0.5f), fmaf(dz, k, -0.5f));
+      if constexpr (ST == PSC_STORAGE_U8 || ST == kStorageU8Far)
+        d = trilinear_quad_u8<32, ST == kStorageU8Far>(u.detail_quad8, fmaf(dx, k, -0.5f), fmaf(dy, k, -0.5f),
+                                                       fmaf(dz, k, -0.5f));
       else
         d = trilinear_texel<ST, 32>(u.noise_detail, fmaf(dx, k, -0.5f), fmaf(dy, k, -0.5f),
                                     fmaf(dz, k, -0.5f), u.noise_scale);

@@ -966,7 +966,10 @@ int launch_march_param_grad(const MarchUniforms& u, const ViewDev& v, const Para
   if (g.layer >= u.layer_count || g.layer >= 8u) return PSC_ERR_INVALID_ARGUMENT;
   cudaError_t e;
   switch (storage) {
-    case PSC_STORAGE_U8: e = launch_st<PSC_STORAGE_U8>(u, v, g, out, loss, s); break;
+    case PSC_STORAGE_U8:
+      e = u.far_texels ? launch_st<kStorageU8Far>(u, v, g, out, loss, s)
+                       : launch_st<PSC_STORAGE_U8>(u, v, g, out, loss, s);
+      break;
     case PSC_STORAGE_F32: e = launch_st<PSC_STORAGE_F32>(u, v, g, out, loss, s); break;
     case PSC_STORAGE_F16: e = launch_st<PSC_STORAGE_F16>(u, v, g, out, loss, s); break;
     case PSC_STORAGE_BF16: e = launch_st<PSC_STORAGE_BF16>(u, v, g, out, loss, s); break;

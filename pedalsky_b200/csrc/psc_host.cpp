@@ -312,6 +312,21 @@ void live_band(const PscCloudLayerGpu& L, psc::LayerConst& o) {
   cache_n = std::min(cache_n + 1, 32u);
 }
 
+// Whether a noise tap of layer L can lie 2^22 texels or more from the origin.
+// Taps are taken inside the layer's shell, whose points are at most
+// R + altitude from the planet's centre at (0, -R, 0), and shifted by the
+// layer's wind and skew and by the curl.  With the default noise scales that is
+// half a million texels and the drift of four months of wind at 10 m/s more.
+bool far_texels(const psc::MarchUniforms& u, const psc::LayerConst& L) {
+  const double wind = std::fabs((double)L.wind_off_x) + std::fabs((double)L.wind_off_z) +
+                      std::fabs((double)L.skew_kx) + std::fabs((double)L.skew_kz);
+  const double reach =
+      2.0 * std::fabs((double)u.planet_r) + std::fabs((double)L.base_m) + std::fabs((double)L.top_m) + wind;
+  const double texels =
+      std::fmax(reach * u.base_texel_scale, reach * u.detail_texel_scale + 32.0 * std::fabs((double)u.curl_strength));
+  return !(texels * 1.001 + 1.0 < 4194304.0);  // not a number: far
+}
+
 void build_uniforms_for(const psc_ctx* c, const PscCloudParamsGpu& p, const PscCloudLayerGpu* layers,
                         const PscFrameUniformsGpu& f, uint32_t width, uint32_t height,
                         psc::MarchUniforms& u) {
@@ -462,6 +477,7 @@ void build_uniforms_for(const psc_ctx* c, const PscCloudParamsGpu& p, const PscC
     live_band(L, o);
     o.r_bottom = (double)w.planet_radius_m + (double)L.base_m;
     o.r_top = (double)w.planet_radius_m + (double)L.top_m;
+    if (i < u.layer_count && far_texels(u, o)) u.far_texels = 1u;
   }
 
   u.noise_base = c->d_base_store;
@@ -841,7 +857,7 @@ int enqueue_batch(psc_ctx* c, uint32_t n, uint32_t n_tiles, cudaStream_t s, bool
   PSC_CUDA(cudaMemsetAsync(c->d_bcounter, 0, sizeof(uint32_t), s), "batch counter reset");
   const int rc = psc::launch_march_batch(c->opts, (int)c->batch_tuning.threads, c->batch_tuning.tile_w,
                                          c->d_bu, c->d_bv, c->d_btiles, n_tiles, c->d_bcounter, c->sms,
-                                         psc::needs_full_paths(c->h_bu, n), s);
+                                         psc::needs_full_paths(c->h_bu, n), psc::any_far_texels(c->h_bu, n), s);
   if (rc == PSC_ERR_UNSUPPORTED)
     return fail(rc, "batched march supports F16/U8/F32 exact, F16/U8 hybrid and U8 texture storage");
   if (rc) return fail(rc, "batched march launch failed: %s", cudaGetErrorString(cudaGetLastError()));
@@ -2152,6 +2168,7 @@ int psc_render_batch(psc_ctx* c, const PscBatchView* views, uint32_t n, void* st
                                (uint64_t)(uintptr_t)c->d_bframes,
                                (uint64_t)(uintptr_t)c->d_base_store, (uint64_t)c->tex_base,
                                (uint64_t)psc::needs_full_paths(c->h_bu, n),
+                               (uint64_t)psc::any_far_texels(c->h_bu, n),
                                fnv1a(c->batch_bake.data(), n)};
   if (per_view) {
     key.push_back(fnv1a(c->h_bu, n * sizeof(psc::MarchUniforms)));

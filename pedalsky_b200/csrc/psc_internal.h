@@ -140,6 +140,7 @@ struct alignas(16) MarchUniforms {
   const uint2* detail_quad;
   const uint4* base_quad8;     // U8
   const uint4* detail_quad8;
+  uint32_t far_texels;         // noise coordinates may pass 2^22 texels (trilinear_quad_u8)
   const uint4* curl_quad;      // FAST schedule: curl tile as 2x2 (R, G) half quads
   // transmittance / sky-view LUTs through the texture unit; 0 = plain loads
   cudaTextureObject_t tex_trans, tex_sky;
@@ -301,10 +302,17 @@ inline __host__ __device__ bool needs_full_paths(const MarchUniforms* u, uint32_
   }
   return false;
 }
-// Persistent batched march (march_batch.cu); `full` as needs_full_paths.
+// True when one of these n uniform blocks is of a scene with far_texels.
+inline bool any_far_texels(const MarchUniforms* u, uint32_t n) {
+  for (uint32_t v = 0; v < n; ++v)
+    if (u[v].far_texels) return true;
+  return false;
+}
+// Persistent batched march (march_batch.cu); `full` as needs_full_paths, `far`
+// as any_far_texels.
 int launch_march_batch(const PscMarchOptions& o, int threads, uint32_t tile_w,
                        const MarchUniforms* u, const ViewDev* v, const uint32_t* tiles,
-                       uint32_t n_tiles, uint32_t* counter, int sms, bool full, cudaStream_t stream);
+                       uint32_t n_tiles, uint32_t* counter, int sms, bool full, bool far, cudaStream_t stream);
 // Per-view sky-view + aerial-perspective LUTs for a batch (atmosphere.cu):
 // `d_frames` holds n frame records built by frame_lite_from; outputs are
 // float4 (RGBA16F-rounded), sky 192x108 and AP 32x32x64 per view.
