@@ -17,21 +17,21 @@
 // Adjoint: one thread per ray runs the forward march, evaluates its pixel's
 // loss term (I - target)^2 / N with I = L + background * T, then walks the
 // steps backwards, carrying the adjoint of the transmittance.  The
-// transmittance before a step is exp(-sigma_t * step * k * prefix), prefix the
-// sum of the grid values of the steps before it: the forward march sums them
-// in FP64 and the reverse sweep takes each step's value off again, each held to
+// transmittance before a step is exp(-sigma_t * k * prefix), prefix the sum of
+// grid value x step over the steps before it: the forward march sums them in
+// FP64 and the reverse sweep takes each step's value off again, each held to
 // what makes a step opaque (`cap`) so that no value is lost beside a larger one
-// (2^-53 of 256 such steps is 1e-11 of optical depth; 1341 -> 1359 us).  Neither
-// checkpoints nor a recomputed segment are needed and the L1 has no shared
-// memory to make room for (checkpoints and segment buffers in 25.6 KB of shared
-// memory per CTA: 1886 us, without: 1668 us; each KB per CTA more cost about 20
-// us).  d loss / d density at the
-// primary sample and d loss / d optical depth toward the sun are scattered
-// into the gradient with vector atomic adds over the trilinear weights of the
-// primary sample and of the six light taps, one 16-byte add per y row (as
-// 8-byte pairs, four per tap, the scatter took 270 us of 1668; now 90 of
-// 1362).  Loss and d loss / d density_scale are reduced per CTA and added in
-// double.
+// (2^-53 of 256 such steps is 1e-11 of optical depth; 1171 us without it, 1173
+// with: the bound comes from the host, found per ray it spilled and took 1.4 %
+// more).  Neither checkpoints nor a recomputed segment are needed and the L1 has
+// no shared memory to make room for (checkpoints and segment buffers in 25.6 KB
+// of shared memory per CTA: 1886 us, without: 1668 us; each KB per CTA more cost
+// about 20 us).  d loss / d density at the primary sample and d loss / d optical
+// depth toward the sun are scattered into the gradient with vector atomic adds
+// over the trilinear weights of the primary sample and of the six light taps,
+// one 16-byte add per y row (as 8-byte pairs, four per tap, the scatter took 270
+// us of 1668; now 90 of 1362).  Loss and d loss / d density_scale are reduced per
+// CTA and added in double.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -217,16 +217,8 @@ __device__ __forceinline__ void grid_pixel(const MarchUniforms& u, const ViewDev
   const bool hit = (rs.hit_mask & 1u) && t1 > t0;
   const float step = hit ? __fdividef(t1 - t0, (float)u.cloud_steps) : 0.0f;
   uint32_t n_exec = 0;
-  double pre = 0.0;  // adjoint: sum of the grid values of the executed steps
-  // adjoint: a grid value is summed up to an optical depth of 200 in the most
-  // transparent channel, where FP32 transmittance is 0 (e^-104 is its least)
-  float cap = 0.0f;
-  if constexpr (ADJ) {
-    float least = INFINITY;
-#pragma unroll
-    for (int c = 0; c < 3; ++c) least = st[c] > 0.0f ? fminf(least, st[c]) : least;
-    cap = 200.0f / (fabsf(g.k) * step * least);
-  }
+  double pre = 0.0;  // adjoint: sum of grid value x step of the executed steps
+  auto summed = [&](float gv) { return (double)fminf(fmaxf(gv * step, -g.cap), g.cap); };
   // an infinity or NaN somewhere in the grid reaches L through the light sum
   // of an empty sample (0 x inf), so such a grid has every sample lit
   const bool every = __ldg(g.nonfinite) != 0u;
@@ -273,7 +265,7 @@ __device__ __forceinline__ void grid_pixel(const MarchUniforms& u, const ViewDev
         if (s >= u.cloud_steps || (gv == 0.0f && !every)) continue;
         const Sample p = position(s);
         const GridPos gp = grid_pos(g, p.x, p.alt, p.z);
-        if constexpr (ADJ) pre += (double)fminf(fmaxf(gv, -cap), cap);
+        if constexpr (ADJ) pre += summed(gv);
         const LightGeo lg = light_geo(u, g, L, gp, p);
         const float gl = light_sum<WIDE>(u, g, lg, p);
         const float rho = g.k * gv, od = g.k * gl;
@@ -324,7 +316,6 @@ __device__ __forceinline__ void grid_pixel(const MarchUniforms& u, const ViewDev
   loss_out = loss;
   float dk = 0.0f;
   if (n_exec > 0) {
-    const float kstep = g.k * step;
     float bT[3] = {T[0], T[1], T[2]};  // transmittance before the step
     for (uint32_t s = n_exec; s-- > 0u;) {
       const Sample p = position(s);
@@ -335,8 +326,8 @@ __device__ __forceinline__ void grid_pixel(const MarchUniforms& u, const ViewDev
       if (!in && !every) continue;
       const float gv = grid_fetch<WIDE>(g, cell);
       if (gv != 0.0f || every) {
-        pre -= (double)fminf(fmaxf(gv, -cap), cap);
-        const float p_od = kstep * (float)pre;  // optical depth per unit sigma_t before the step
+        pre -= summed(gv);
+        const float p_od = g.k * (float)pre;  // optical depth per unit sigma_t before the step
 #pragma unroll
         for (int c = 0; c < 3; ++c) bT[c] = __expf(-st[c] * p_od);
       }

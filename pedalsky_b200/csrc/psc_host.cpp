@@ -2529,6 +2529,9 @@ int prepare_grid(psc_ctx* c, const PscDensityGrid* g, const PscView* v, bool adj
   gd.inv_cell_y = (float)g->ny / std::max(L.top_m - L.base_m, 1.0f);
   gd.inv_sigma_bar = 3.0f / sig;
   gd.k = g->density_scale * gd.inv_sigma_bar;
+  float least = INFINITY;
+  for (const float st : L.sigma_t) least = st > 0.0f ? std::min(least, st) : least;
+  gd.cap = 200.0f / (std::fabs(gd.k) * least);
   gd.exit_t = g->exit_transmittance;
   gd.inv_n = (float)(1.0 / (3.0 * (double)vw * (double)vh));
   return PSC_OK;

@@ -166,6 +166,10 @@ struct GridDev {
   float min_x, min_z, base;
   float inv_cell_x, inv_cell_y, inv_cell_z;
   float k;                 // density = k * value (density_scale * inv_sigma_bar)
+  // adjoint: a step's grid value x length is summed up to an optical depth of
+  // 200 in the most transparent channel, where FP32 transmittance is 0 (e^-104
+  // is its least)
+  float cap;
   float inv_sigma_bar;     // 3 / (sigma_t.r + sigma_t.g + sigma_t.b) of layer 0
   float exit_t;            // early exit once max(T) < exit_t
   float inv_n;             // 1 / (3 * viewport pixels)
