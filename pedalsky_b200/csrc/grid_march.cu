@@ -424,9 +424,11 @@ __global__ void __launch_bounds__(kThreads, MINB) k_grid_march(const __grid_cons
 
 // One warp per (yi, zi) row of quads, so no index is divided per quad.  Sets
 // *nonfinite when a value is an infinity or NaN.
-__global__ void __launch_bounds__(256) k_grid_quads(const __grid_constant__ GridDev g, float4* __restrict__ q,
+// Bounded by its writes; 8 blocks per SM (32 registers), as many as are launched,
+// keep it one wave: at 34 registers a grid_512 call takes 1 to 3 us more of 240.
+__global__ void __launch_bounds__(256, 8) k_grid_quads(const __grid_constant__ GridDev g, float4* __restrict__ q,
                                                     uint32_t* __restrict__ nonfinite) {
-  const uint32_t lane = threadIdx.x & 31u, pad = g.pad, sx = g.row, sz = (uint32_t)(g.plane / sx);
+  const uint32_t lane = threadIdx.x & 31u, pad = g.pad, sx = g.row, sz = g.nz + 2u * pad - 1u;
   const uint64_t rows = (uint64_t)(g.ny + 2u * g.pad_y) * sz, warps = (uint64_t)gridDim.x * (blockDim.x >> 5);
   bool bad = false;
   for (uint64_t row = (uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); row < rows; row += warps) {
