@@ -102,7 +102,9 @@ struct Sample {
 // Light march of one sample (cloud_march.wgsl:543-578) in grid coordinates:
 // x and z are affine along the sun ray, and for light paths up to 20 km the
 // altitude is the cubic of march_fast_body.cuh's LightRay (truncation below
-// 1e-4 m); longer ones take the altitude of each tap from the geometry.
+// 1e-4 m; with its rounding off by 2.1e-4 m rms, 1.0e-3 at most, over paths of
+// all lengths, the geometry's form by 2.2e-4 and 1.25e-3); longer ones take the
+// altitude of each tap from the geometry.
 struct LightGeo {
   float x, z, kx, kz;    // x + kx t, z + kz t
   float c0, c1, c2, c3;  // y = c0 + t (c1 + t (c2 + t c3))
